@@ -265,9 +265,16 @@ def build_replay_state(problem, y0, params, *, method: str, rtol: float, atol: f
     spec, y0_t, p_t, pk = _prepare(problem, y0, params, dev)
     t1s, t1v = _t1_arg(problem, t1, dev)
     ms = int(max_steps or 100000)
+    # ("sqrt" takes its interval from the capacity, so it keeps the default one)
+    cap0, budget = engine.DEFAULT_CAP0, None
+    if checkpoint != "sqrt":
+        budget = engine._checkpoint_budget()
+        K = (checkpoint if isinstance(checkpoint, int) else 1 if checkpoint == "all" else
+             engine.tuned_ckpt_every(method, spec, precision) or 2)
+        cap0 = engine.first_capacity(y0_t.shape[0], spec.dim, ms, K, precision, budget)
     r = engine.forward_record(method, spec, y0_t, pk, t0=float(problem.t0), t1=t1s, t1v=t1v,
-                              rtol=rtol, atol=atol, max_steps=ms, checkpoint=checkpoint,
-                              precision=precision,
+                              rtol=rtol, atol=atol, max_steps=ms, cap0=cap0,
+                              checkpoint=checkpoint, budget_bytes=budget, precision=precision,
                               # the float32 route records without dense output: its closure
                               # replays the saved states at the recording point
                               saveat_ts=None if precision == "float32" else saveat)

@@ -116,6 +116,33 @@ def choose_ckpt_every(policy, dim: int, n: int, cap: int, budget_bytes: Optional
     return min(K, kmax)
 
 
+# A record that starts at DEFAULT_CAP0 steps re-solves the trajectories that outgrow it, from
+# their start, in further tiers: the stiff Van der Pol batch of 20,011 trajectories (2269 steps on
+# average, 17,220 the longest) ran four forwards one after another, 1024 + 4096 + 16384 + 17220
+# attempts on the critical path instead of 17,220.  Where the whole batch fits a sixteenth of the
+# free memory at a larger capacity, the first record takes that capacity: only the slots that
+# are written are touched, so the forward is as fast, and nothing is solved twice.  A small
+# share, because the buffers live as long as their closure: large batches stay at DEFAULT_CAP0
+# (2^18 trajectories of 3 components reach a sixteenth of 180 GB at 1780 steps).
+CAP_SHARE = 4  # of the checkpoint budget, itself a quarter of the free memory
+
+
+def first_capacity(n: int, dim: int, max_steps: int, ckpt_every: int, precision: str,
+                   budget_bytes: Optional[int] = None) -> int:
+    """Steps per trajectory of a fresh record: at least DEFAULT_CAP0, at most max_steps, and
+    in between as many as keep the record and its checkpoints every ``ckpt_every`` steps within
+    1/CAP_SHARE of the checkpoint budget."""
+    lo = max(1, min(DEFAULT_CAP0, int(max_steps)))
+    if n <= 0 or lo >= int(max_steps):
+        return lo
+    if budget_bytes is None:
+        budget_bytes = _checkpoint_budget()
+    word, row = ((4, 4 * ckpt_width_f32(dim)) if precision == "float32" else
+                 (8, 8 * ckpt_width(dim)))
+    per_step = n * (word + -(-row // ckpt_every))
+    return max(lo, min(int(max_steps), budget_bytes // CAP_SHARE // per_step - 2 * ckpt_every))
+
+
 # ---- checkpoint-interval autotuner ---------------------------------------------------------
 # The reverse pass keeps each thread's K segment states (and, for Tsit5 float64, their stage
 # inputs) in shared memory, so K trades recomputation and checkpoint traffic (none and the
@@ -992,7 +1019,11 @@ def _forward_planned(method, spec, y0, p, t1v, saveat_ts, ws: RecordSet, kw):
 def raise_on_failed(r: Record, max_steps: int, t1) -> None:
     """Refuse an incomplete mesh, with the reference's messages
     (gradsolve/warp/warp_replay.py:167-173, gradsolve/solvers/record_jax.py:201-211)."""
-    if r.n == 0 or r.status_max == 0:  # (the forward's own check read every status)
+    if r.n == 0:
+        return
+    if r.status_max is None:  # (a record of max_steps capacity: the forward read no status)
+        r.status_max = _status_max(r.status, r.status.device)
+    if r.status_max == 0:
         return
     bad = torch.nonzero(r.status != 0).flatten()
     if bad.numel() == 0:
