@@ -701,11 +701,12 @@ int launch_ros23_adjoint(const gs::AdjointArgs& a, int cap, cudaStream_t s, int 
   if (sched == GS_SCHED_STATIC) {
     SegCfg ck{0, 0, 0}, cr{0, 0, 0};
     int rc;
-    if ((rc = occupancy_probe(gs::ros23_adjoint_kernel<F, true>,
-                              gs::ros23_adjoint_smem_doubles<F::D, true>(a.ck_every), &ck)))
-      return rc;
     if ((rc = occupancy_probe(gs::ros23_adjoint_kernel<F, false>,
                               gs::ros23_adjoint_smem_doubles<F::D, false>(a.ck_every), &cr)))
+      return rc;
+    if constexpr (!gs::kSparseW<F, double>) {  // (a sparse W is cheaper to refactor than to keep)
+    if ((rc = occupancy_probe(gs::ros23_adjoint_kernel<F, true>,
+                              gs::ros23_adjoint_smem_doubles<F::D, true>(a.ck_every), &ck)))
       return rc;
     if (keeping_pays(ck, cr)) {
       auto keep = gs::ros23_adjoint_kernel<F, true>;
@@ -726,6 +727,7 @@ int launch_ros23_adjoint(const gs::AdjointArgs& a, int cap, cudaStream_t s, int 
       if ((rc = allow_smem(keep, ck.smem))) return rc;
       keep<<<grid_for_block(a.n, ck.block), ck.block, ck.smem, s>>>(a);
       return cuda_check("ros23_adjoint_kernel");
+    }
     }
     // large K: the kept factors would cost too many resident threads (or not fit); recompute
     if (cr.resident <= 0)

@@ -133,7 +133,7 @@ __device__ __forceinline__ bool tsit5_coop_attempt(const RecordArgs& a, long lon
     const double e = h * (T::E1 * k1[i] + T::E2 * S.k2[i] + T::E3 * S.k3[i] + T::E4 * S.k4[i] +
                           T::E5 * S.k5[i] + T::E6 * S.k6[i] + T::E7 * ko[i]);
     const double sc = a.atol + a.rtol * fmax(fabs(y[i]), fabs(yo[i]));
-    const double q = e / sc;
+    const double q = e * reciprocal(sc);
     part += q * q;
   }
   const double m = L::sum(part);

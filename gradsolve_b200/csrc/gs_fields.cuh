@@ -37,6 +37,8 @@
 //   vjp(y, p, w, gy, gp)          gy += (df/dy)^T w, gp += (df/dp)^T w
 //   jac(y, p, J)                  J = df/dy, row-major D x D          (stiff fields)
 //   jac_contract_grad(y,p,G,gy,gp) gy += d/dy <G, J(y,p)>, gp += d/dp <G, J(y,p)>
+//   jac_nz(i, c)                  false where J[i][c] is 0 for every (y, p): the Rosenbrock23
+//                                 kernels leave those entries out (without it: none is)
 #pragma once
 
 namespace gs {
@@ -156,6 +158,7 @@ struct VdP {
     gy[1] += w[0] + w[1] * mu * (R(1.0) - x * x);
     gp[0] += w[1] * ((R(1.0) - x * x) * v - x);
   }
+  static constexpr GS_HD bool jac_nz(int i, int c) { return i != 0 || c != 0; }
   // J = [[0, 1], [mu (-2 x v - 1), mu (1 - x^2)]]  (for Rosenbrock23 at large mu)
   template <class R>
   static GS_HD void jac(const R* y, const R* p, R* J) {
@@ -232,6 +235,7 @@ struct Linear {
 #pragma unroll
     for (int i = 0; i < D; ++i) gy[i] += R(1.01) * w[i];
   }
+  static constexpr GS_HD bool jac_nz(int i, int c) { return i == c; }
   template <class R>
   static GS_HD void jac(const R*, const R*, R* J) {
 #pragma unroll
@@ -333,6 +337,10 @@ struct Hires {
     gy[6] += R(0.43) * w[4] + R(0.69) * w[5] - R(1.81) * w[6] + R(1.81) * w[7];
     gy[7] += R(-280.0) * y[5] * w[5] + R(280.0) * y[5] * w[6] - R(280.0) * y[5] * w[7];
   }
+  // the entries jac writes
+  static constexpr GS_HD bool jac_nz(int i, int c) {
+    return (0xe0e0f8700e1c0307ull >> (8 * i + c)) & 1;
+  }
   template <class R>
   static GS_HD void jac(const R* y, const R*, R* J) {
 #pragma unroll
@@ -409,6 +417,7 @@ struct Robertson {
     gp[1] += -b * b * w[1] + b * b * w[2];
     gp[2] += b * c * w[0] - b * c * w[1];
   }
+  static constexpr GS_HD bool jac_nz(int i, int c) { return i != 2 || c == 1; }
   template <class R>
   static GS_HD void jac(const R* y, const R* p, R* J) {
     const R k1 = p[0], k2 = p[1], k3 = p[2], b = y[1], c = y[2];

@@ -124,17 +124,9 @@ struct LaneRos23 {
   __device__ __forceinline__ void start(const double*, const double*, const float*) {}
   __device__ __forceinline__ double trial(const double* y, const double* p, const float*, double h,
                                           double rtol, double atol, double* ynew) {
-    RosCore<F> c;
-    ros23_core<F>(y, p, h, c, ynew);
-    double F2[D], r3[D], k3[D], ev[D];
-    F::rhs(ynew, p, F2);
-#pragma unroll
-    for (int i = 0; i < D; ++i)
-      r3[i] = F2[i] - Ros23::E32 * (c.k2[i] - c.F1[i]) - 2.0 * (c.k1[i] - c.F0[i]);
-    lu_solve<D>(c.W, r3, k3);
-#pragma unroll
-    for (int i = 0; i < D; ++i) ev[i] = (h / 6.0) * (c.k1[i] - 2.0 * c.k2[i] + k3[i]);
-    return wrms_sumsq<D>(ev, y, ynew, rtol, atol);
+    double ev[D];
+    ros23_trial<F>(y, p, h, ynew, ev);
+    return wrms_sumsq<D, false>(ev, y, ynew, rtol, atol);
   }
   __device__ __forceinline__ void commit() {}
   // the step no longer advances time: status 2 (gradsolve/solvers/record_jax.py:109)
@@ -152,10 +144,6 @@ struct LaneRos23 {
 // A saveat re-step, out of line: re-steps are rare (a few per trajectory against thousands of
 // attempts), and inlined, the step's temporaries would raise the register count of the whole
 // attempt loop.  Arguments and result travel by value (no address of a register array).
-template <int N>
-struct DVec {
-  double v[N];
-};
 template <int N>
 struct FVec {
   float v[N];

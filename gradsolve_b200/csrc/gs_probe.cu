@@ -62,3 +62,18 @@ extern "C" int gs_probe_step_factor(const double* S, long long n, int order, int
       S, n, order, D, c, fast, ref, accept_fast, accept_ref);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
+
+// ---- the solver's reciprocal against the division ----------------------------------------
+__global__ void reciprocal_probe(const double* x, long long n, double* r, double* ref) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  r[i] = gs::reciprocal(x[i]);
+  ref[i] = 1.0 / x[i];
+}
+
+extern "C" int gs_probe_reciprocal(const double* x, long long n, double* r, double* ref,
+                                   void* stream) {
+  if (n <= 0) return 0;
+  reciprocal_probe<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, n, r, ref);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}

@@ -47,27 +47,81 @@ struct LU {
   int piv[D];       // (LU only)
 };
 
-template <int D, class R>
-__device__ __forceinline__ void inverse_factor(LU<D, R>& f) {
+// The entries of W = I - d h J that are not 0 for every (y, p) (F::jac_nz; all of them for a
+// field that does not say).
+template <class F, class = void>
+struct jac_pattern {
+  static constexpr GS_HD bool nz(int, int) { return true; }
+};
+template <class F>
+struct jac_pattern<F, decltype(void(F::jac_nz(0, 0)))> {
+  static constexpr GS_HD bool nz(int i, int c) { return F::jac_nz(i, c); }
+};
+
+// ... as bit masks (bit i * D + c), for D <= 8: kW of W itself, kLU of L and U eliminated without
+// row exchanges, fill-in included.
+template <class F>
+constexpr unsigned long long w_mask(bool eliminated) {
+  constexpr int D = F::D;
+  unsigned long long m = 0;
+  if (D > 8) return ~0ull;
+  for (int i = 0; i < D; ++i)
+    for (int c = 0; c < D; ++c)
+      if (i == c || jac_pattern<F>::nz(i, c)) m |= 1ull << (i * D + c);
+  for (int k = 0; eliminated && k < D; ++k)
+    for (int r = k + 1; r < D; ++r)
+      for (int c = k + 1; c < D; ++c)
+        if (((m >> (r * D + k)) & 1) && ((m >> (k * D + c)) & 1)) m |= 1ull << (r * D + c);
+  return m;
+}
+template <class F>
+constexpr unsigned long long kW = w_mask<F>(false);
+template <class F>
+constexpr unsigned long long kLU = w_mask<F>(true);
+
+constexpr int bit_count(unsigned long long m) {
+  int k = 0;
+  for (; m; m &= m - 1) ++k;
+  return k;
+}
+
+// x1 x2 - y1 y2 where kX / kY say which products are not 0 for every (y, p)
+template <bool kX, bool kY, class R>
+__device__ __forceinline__ R minor2(R x1, R x2, R y1, R y2) {
+  if constexpr (kX && kY) return x1 * x2 - y1 * y2;
+  if constexpr (kX && !kY) return x1 * x2;
+  if constexpr (!kX && kY) return -(y1 * y2);
+  return R(0.0);
+}
+
+// W^-1 by cofactors (kInverseW); products with an entry that is 0 by the field's pattern are
+// left out (a diagonal entry without a Jacobian term is the literal 1).
+template <class F, class R>
+__device__ __forceinline__ void inverse_factor(LU<F::D, R>& f) {
+  constexpr int D = F::D;
+#define GS_W(i) (bool)((kW<F> >> (i)) & 1)
   R* a = f.a;
   if constexpr (D == 1) {
-    a[0] = R(1.0) / a[0];
+    a[0] = reciprocal(a[0]);
   } else if constexpr (D == 2) {
-    const R r = R(1.0) / (a[0] * a[3] - a[1] * a[2]);
     const R a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3];
+    const R r = reciprocal(minor2<true, GS_W(1) && GS_W(2)>(a0, a3, a1, a2));
     a[0] = a3 * r;
     a[1] = -a1 * r;
     a[2] = -a2 * r;
     a[3] = a0 * r;
   } else {
     // cofactors c_ij of W; W^-1 = adj(W) / det = (c_ji) / det
-    const R c00 = a[4] * a[8] - a[5] * a[7], c01 = a[5] * a[6] - a[3] * a[8],
-            c02 = a[3] * a[7] - a[4] * a[6];
-    const R c10 = a[2] * a[7] - a[1] * a[8], c11 = a[0] * a[8] - a[2] * a[6],
-            c12 = a[1] * a[6] - a[0] * a[7];
-    const R c20 = a[1] * a[5] - a[2] * a[4], c21 = a[2] * a[3] - a[0] * a[5],
-            c22 = a[0] * a[4] - a[1] * a[3];
-    const R r = R(1.0) / (a[0] * c00 + a[1] * c01 + a[2] * c02);
+#define GS_MINOR(i, j, k, l) \
+  minor2<GS_W(i) && GS_W(j), GS_W(k) && GS_W(l)>(a[i], a[j], a[k], a[l])
+    const R c00 = GS_MINOR(4, 8, 5, 7), c01 = GS_MINOR(5, 6, 3, 8), c02 = GS_MINOR(3, 7, 4, 6);
+    const R c10 = GS_MINOR(2, 7, 1, 8), c11 = GS_MINOR(0, 8, 2, 6), c12 = GS_MINOR(1, 6, 0, 7);
+    const R c20 = GS_MINOR(1, 5, 2, 4), c21 = GS_MINOR(2, 3, 0, 5), c22 = GS_MINOR(0, 4, 1, 3);
+#undef GS_MINOR
+    R det = a[0] * c00;
+    if constexpr (GS_W(1)) det = det + a[1] * c01;
+    if constexpr (GS_W(2)) det = det + a[2] * c02;
+    const R r = reciprocal(det);
     a[0] = c00 * r;
     a[1] = c10 * r;
     a[2] = c20 * r;
@@ -78,14 +132,11 @@ __device__ __forceinline__ void inverse_factor(LU<D, R>& f) {
     a[7] = c12 * r;
     a[8] = c22 * r;
   }
+#undef GS_W
 }
 
 template <int D, class R>
 __device__ __forceinline__ void lu_factor(LU<D, R>& f) {
-  if constexpr (kInverseW<D, R>) {
-    inverse_factor(f);
-    return;
-  }
 #pragma unroll
   for (int col = 0; col < D; ++col) {
     int pv = col;
@@ -215,18 +266,119 @@ __device__ __forceinline__ void lu_solve_t(const LU<D, R>& f, const R* b, R* x) 
   }
 }
 
-template <class F, class R = double>
-__device__ __forceinline__ void ros23_build_w(const R* y, const R* p, R h, LU<F::D, R>& W) {
+template <class F, class R>
+__device__ __forceinline__ void ros23_w(const R* y, const R* p, R h, R* W) {
   constexpr int D = F::D;
   R J[D * D];
   F::jac(y, p, J);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
 #pragma unroll
-    for (int c = 0; c < D; ++c) W.a[i * D + c] = -R(Ros23::D) * h * J[i * D + c];
-    W.a[i * D + i] = W.a[i * D + i] + R(1.0);
+    for (int c = 0; c < D; ++c)
+      W[i * D + c] = jac_pattern<F>::nz(i, c) ? -R(Ros23::D) * h * J[i * D + c] : R(0.0);
+    W[i * D + i] = jac_pattern<F>::nz(i, i) ? W[i * D + i] + R(1.0) : R(1.0);
   }
-  lu_factor(W);
+}
+
+template <class F, class R = double>
+__device__ __forceinline__ void ros23_build_w(const R* y, const R* p, R h, LU<F::D, R>& W) {
+  ros23_w<F>(y, p, h, W.a);
+  if constexpr (kInverseW<F::D, R>) {
+    inverse_factor<F>(W);
+  } else {
+    lu_factor(W);
+  }
+}
+
+// Float64 fields of 4 to 8 components whose W stays sparse under elimination (at most 5/8 of
+// the entries with the fill-in): the elimination and the solves run over the nonzero entries
+// alone, unrolled from the pattern at compile time, on the diagonal's pivots.  sparse_factor
+// returns false where partial pivoting would take another row somewhere; the caller then runs
+// the step out of line with the pivoted elimination over all entries, so the pivots are those
+// of the reference's elimination either way and the values differ by the rounding of a
+// pivot's reciprocal alone.  HIRES (33 of 64 entries): the pivoted elimination with its
+// searches, row selects and three dense solves kept one warp per scheduler at 255 registers and
+// 3.66 us per attempt.
+template <class F, class R>
+constexpr bool kSparseW = F::D > 3 && F::D <= 8 && std::is_same<R, double>::value &&
+                          bit_count(kLU<F>) * 8 <= F::D * F::D * 5;
+
+template <class F>
+__device__ __forceinline__ bool sparse_factor(LU<F::D>& f) {
+  constexpr int D = F::D;
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    f.inv[k] = reciprocal(f.a[k * D + k]);
+#pragma unroll
+    for (int r = k + 1; r < D; ++r) {
+      if (((kLU<F> >> (r * D + k)) & 1)) {
+        ok = ok && !(fabs(f.a[r * D + k]) > fabs(f.a[k * D + k]));
+        const double factor = f.a[r * D + k] * f.inv[k];
+        f.a[r * D + k] = factor;
+#pragma unroll
+        for (int c = k + 1; c < D; ++c)
+          if (((kLU<F> >> (k * D + c)) & 1)) f.a[r * D + c] = f.a[r * D + c] - factor * f.a[k * D + c];
+      }
+    }
+  }
+  return ok;
+}
+
+template <class F>
+__device__ __forceinline__ void sparse_solve(const LU<F::D>& f, const double* b, double* x) {
+  constexpr int D = F::D;
+#pragma unroll
+  for (int i = 0; i < D; ++i) x[i] = b[i];
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+#pragma unroll
+    for (int r = k + 1; r < D; ++r)
+      if (((kLU<F> >> (r * D + k)) & 1)) x[r] = x[r] - f.a[r * D + k] * x[k];
+  }
+#pragma unroll
+  for (int i = D - 1; i >= 0; --i) {
+    double s = x[i];
+#pragma unroll
+    for (int c = i + 1; c < D; ++c)
+      if (((kLU<F> >> (i * D + c)) & 1)) s = s - f.a[i * D + c] * x[c];
+    x[i] = s * f.inv[i];
+  }
+}
+
+template <class F>
+__device__ __forceinline__ void sparse_solve_t(const LU<F::D>& f, const double* b, double* x) {
+  constexpr int D = F::D;
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    double s = b[i];
+#pragma unroll
+    for (int k = 0; k < i; ++k)
+      if (((kLU<F> >> (k * D + i)) & 1)) s = s - f.a[k * D + i] * x[k];
+    x[i] = s * f.inv[i];
+  }
+#pragma unroll
+  for (int i = D - 1; i >= 0; --i) {
+    double s = x[i];
+#pragma unroll
+    for (int r = i + 1; r < D; ++r)
+      if (((kLU<F> >> (r * D + i)) & 1)) s = s - f.a[r * D + i] * x[r];
+    x[i] = s;
+  }
+}
+
+// x = W^-1 b (kT: W^-T b) from the factors of ros23_core; kSparse: those of sparse_factor.
+template <class F, bool kSparse, bool kT, class R>
+__device__ __forceinline__ void w_solve(const LU<F::D, R>& W, const R* b, R* x) {
+  if constexpr (kSparse && kT) {
+    sparse_solve_t<F>(W, b, x);
+  } else if constexpr (kSparse) {
+    sparse_solve<F>(W, b, x);
+  } else if constexpr (kT) {
+    lu_solve_t(W, b, x);
+  } else {
+    lu_solve(W, b, x);
+  }
 }
 
 // Shared part of the attempt and of the replay step: W factored, F0, k1, F1, k2, ynew.
@@ -237,24 +389,108 @@ struct RosCore {
   R F0[D], k1[D], F1[D], k2p[D], k2[D];  // k2 = k2p + k1
 };
 
-template <class F, class R = double>
-__device__ __forceinline__ void ros23_core(const R* y, const R* p, R h, RosCore<F, R>& c,
-                                           R* ynew) {
+// kSparse: W by sparse_factor; false where its pivots are not the partial-pivoting ones (the
+// outputs are then not to be used).
+template <class F, bool kSparse, class R>
+__device__ __forceinline__ bool ros23_core_as(const R* y, const R* p, R h, RosCore<F, R>& c,
+                                              R* ynew) {
   constexpr int D = F::D;
   R s[D];
-  ros23_build_w<F>(y, p, h, c.W);
+  bool ok = true;
+  if constexpr (kSparse) {
+    ros23_w<F>(y, p, h, c.W.a);
+    ok = sparse_factor<F>(c.W);
+  } else {
+    ros23_build_w<F>(y, p, h, c.W);
+  }
   F::rhs(y, p, c.F0);
-  lu_solve(c.W, c.F0, c.k1);
+  w_solve<F, kSparse, false>(c.W, c.F0, c.k1);
 #pragma unroll
   for (int i = 0; i < D; ++i) s[i] = y[i] + R(0.5) * h * c.k1[i];
   F::rhs(s, p, c.F1);
 #pragma unroll
   for (int i = 0; i < D; ++i) s[i] = c.F1[i] - c.k1[i];
-  lu_solve(c.W, s, c.k2p);
+  w_solve<F, kSparse, false>(c.W, s, c.k2p);
 #pragma unroll
   for (int i = 0; i < D; ++i) c.k2[i] = c.k2p[i] + c.k1[i];
 #pragma unroll
   for (int i = 0; i < D; ++i) ynew[i] = y[i] + h * c.k2[i];
+  return ok;
+}
+
+template <class F, class R = double>
+__device__ __forceinline__ void ros23_core(const R* y, const R* p, R h, RosCore<F, R>& c,
+                                           R* ynew) {
+  ros23_core_as<F, false>(y, p, h, c, ynew);
+}
+
+// Vectors by value, for the out-of-line steps (no address of a register array is taken).
+template <int N>
+struct DVec {
+  double v[N];
+};
+template <int N>
+__device__ __forceinline__ DVec<N> to_dvec(const double* a) {
+  DVec<N> r;
+#pragma unroll
+  for (int i = 0; i < N; ++i) r.v[i] = a[i];
+  return r;
+}
+template <int N>
+__device__ __forceinline__ void from_dvec(const DVec<N>& r, double* a) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) a[i] = r.v[i];
+}
+
+// One attempt of the adaptive forward: the candidate yo and the error vector ev.
+template <class F, bool kSparse>
+__device__ __forceinline__ bool ros23_trial_as(const double* y, const double* p, double h,
+                                               double* yo, double* ev) {
+  constexpr int D = F::D;
+  RosCore<F> rc;
+  const bool ok = ros23_core_as<F, kSparse>(y, p, h, rc, yo);
+  double F2[D], r3[D], k3[D];
+  F::rhs(yo, p, F2);
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+    r3[i] = F2[i] - Ros23::E32 * (rc.k2[i] - rc.F1[i]) - 2.0 * (rc.k1[i] - rc.F0[i]);
+  w_solve<F, kSparse, false>(rc.W, r3, k3);
+#pragma unroll
+  for (int i = 0; i < D; ++i) ev[i] = (h / 6.0) * (rc.k1[i] - 2.0 * rc.k2[i] + k3[i]);
+  return ok;
+}
+
+template <class F>
+__device__ __noinline__ DVec<2 * F::D> ros23_trial_pivoted(DVec<F::D> y, DVec<F::P> p, double h) {
+  DVec<2 * F::D> r;
+  ros23_trial_as<F, false>(y.v, p.v, h, r.v, r.v + F::D);
+  return r;
+}
+
+template <class F>
+__device__ __forceinline__ void ros23_trial(const double* y, const double* p, double h,
+                                            double* yo, double* ev) {
+  constexpr int D = F::D;
+  if constexpr (kSparseW<F, double>) {
+    if (!ros23_trial_as<F, true>(y, p, h, yo, ev)) {
+      const DVec<2 * D> r = ros23_trial_pivoted<F>(to_dvec<D>(y), to_dvec<F::P>(p), h);
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        yo[i] = r.v[i];
+        ev[i] = r.v[D + i];
+      }
+    }
+  } else {
+    ros23_trial_as<F, false>(y, p, h, yo, ev);
+  }
+}
+
+template <class F>
+__device__ __noinline__ DVec<F::D> ros23_step_pivoted(DVec<F::D> y, DVec<F::P> p, double dt) {
+  RosCore<F> c;
+  DVec<F::D> yn;
+  ros23_core<F>(y.v, p.v, dt, c, yn.v);
+  return yn;
 }
 
 template <class F, class R = double>
@@ -262,14 +498,19 @@ __device__ __forceinline__ void ros23_replay_step(R* y, const R* p, R dt) {
   constexpr int D = F::D;
   RosCore<F, R> c;
   R yn[D];
-  ros23_core<F>(y, p, dt, c, yn);
+  if constexpr (kSparseW<F, R>) {
+    if (!ros23_core_as<F, true>(y, p, dt, c, yn))
+      from_dvec<D>(ros23_step_pivoted<F>(to_dvec<D>(y), to_dvec<F::P>(p), dt), yn);
+  } else {
+    ros23_core<F>(y, p, dt, c, yn);
+  }
 #pragma unroll
   for (int i = 0; i < D; ++i) y[i] = yn[i];
 }
 
 // Reverse of one replay step from the step's forward quantities: the factors of W, k1, the
 // stage state s1 = y + dt/2 k1 and k2' = W \ (f(s1) - k1).
-template <class F, class R = double>
+template <class F, class R = double, bool kSparse = false>
 __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, const LU<F::D, R>& W,
                                                const R* k1, const R* s1, const R* k2p, R* lam,
                                                R* gp) {
@@ -282,7 +523,7 @@ __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, con
     k1b[i] = k2b[i];
     s1b[i] = R(0.0);
   }
-  lu_solve_t(W, k2b, r2b);
+  w_solve<F, kSparse, true>(W, k2b, r2b);
   const R scale = R(Ros23::D) * dt;  // G = -d dt Wbar, Wbar = -(r2b k2p^T + r1b k1^T)
 #pragma unroll
   for (int i = 0; i < D; ++i) {
@@ -296,7 +537,7 @@ __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, con
     yb[i] += s1b[i];
     k1b[i] += R(0.5) * dt * s1b[i];
   }
-  lu_solve_t(W, k1b, r1b);
+  w_solve<F, kSparse, true>(W, k1b, r1b);
 #pragma unroll
   for (int i = 0; i < D; ++i)
 #pragma unroll
@@ -309,8 +550,8 @@ __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, con
 
 // Reverse of one replay step at (y, dt), recomputing its forward quantities (the expressions
 // of ros23_core).
-template <class F, class R = double>
-__device__ __forceinline__ void ros23_step_vjp(const R* y, const R* p, R dt, R* lam, R* gp) {
+template <class F, class R>
+__device__ __forceinline__ void ros23_step_vjp_dense(const R* y, const R* p, R dt, R* lam, R* gp) {
   constexpr int D = F::D;
   RosCore<F, R> c;
   R yn[D], s1[D];
@@ -318,6 +559,42 @@ __device__ __forceinline__ void ros23_step_vjp(const R* y, const R* p, R dt, R* 
 #pragma unroll
   for (int i = 0; i < D; ++i) s1[i] = y[i] + R(0.5) * dt * c.k1[i];
   ros23_vjp_core<F>(y, p, dt, c.W, c.k1, s1, c.k2p, lam, gp);
+}
+
+template <class F>
+__device__ __noinline__ DVec<F::D + F::P> ros23_step_vjp_pivoted(DVec<F::D> y, DVec<F::P> p,
+                                                                 double dt, DVec<F::D> lam,
+                                                                 DVec<F::P> gp) {
+  DVec<F::D + F::P> r;
+#pragma unroll
+  for (int i = 0; i < F::D; ++i) r.v[i] = lam.v[i];
+#pragma unroll
+  for (int i = 0; i < F::P; ++i) r.v[F::D + i] = gp.v[i];
+  ros23_step_vjp_dense<F>(y.v, p.v, dt, r.v, r.v + F::D);
+  return r;
+}
+
+template <class F, class R = double>
+__device__ __forceinline__ void ros23_step_vjp(const R* y, const R* p, R dt, R* lam, R* gp) {
+  constexpr int D = F::D, P = F::P;
+  if constexpr (kSparseW<F, R>) {
+    RosCore<F, R> c;
+    R yn[D], s1[D];
+    if (ros23_core_as<F, true>(y, p, dt, c, yn)) {
+#pragma unroll
+      for (int i = 0; i < D; ++i) s1[i] = y[i] + R(0.5) * dt * c.k1[i];
+      ros23_vjp_core<F, R, true>(y, p, dt, c.W, c.k1, s1, c.k2p, lam, gp);
+    } else {
+      const DVec<D + P> r = ros23_step_vjp_pivoted<F>(to_dvec<D>(y), to_dvec<P>(p), dt,
+                                                      to_dvec<D>(lam), to_dvec<P>(gp));
+#pragma unroll
+      for (int i = 0; i < D; ++i) lam[i] = r.v[i];
+#pragma unroll
+      for (int i = 0; i < P; ++i) gp[i] = r.v[D + i];
+    }
+  } else {
+    ros23_step_vjp_dense<F>(y, p, dt, lam, gp);
+  }
 }
 
 // One attempt from the state y; the candidate is computed into yo.  Returns true when the
@@ -336,17 +613,9 @@ __device__ __forceinline__ bool ros23_attempt(const RecordArgs& a, long long j, 
     return false;
   }
   ++c.it;
-  RosCore<F> rc;
-  ros23_core<F>(y, p, h, rc, yo);
-  double F2[D], r3[D], k3[D], ev[D];
-  F::rhs(yo, p, F2);
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-    r3[i] = F2[i] - Ros23::E32 * (rc.k2[i] - rc.F1[i]) - 2.0 * (rc.k1[i] - rc.F0[i]);
-  lu_solve<D>(rc.W, r3, k3);
-#pragma unroll
-  for (int i = 0; i < D; ++i) ev[i] = (h / 6.0) * (rc.k1[i] - 2.0 * rc.k2[i] + k3[i]);
-  const double m = wrms_sumsq<D>(ev, y, yo, a.rtol, a.atol);
+  double ev[D];
+  ros23_trial<F>(y, p, h, yo, ev);
+  const double m = wrms_sumsq<D, false>(ev, y, yo, a.rtol, a.atol);
   if (!(m == m)) {
     c.st = 1;
     return false;
@@ -459,8 +728,9 @@ __global__ void __launch_bounds__(128) ros23_replay_kernel(const ReplayArgs a) {
 // prefetched (cp.async) into the shared-memory segment buffer, and the segment's replay keeps
 // what the step VJPs need -- the factors of W (D^2 + 2D values), k1, s1 and k2' -- for the
 // K-1 steps it takes, so only the segment's last step recomputes its forward quantities.
-// kKeep = false (where the kept quantities would not fit shared memory): every step's VJP
-// recomputes them, and the buffer holds only the states, dts and checkpoints.
+// kKeep = false (where the kept quantities would not fit shared memory, and for fields with a
+// sparse W, whose factors cost less to recompute than to keep): every step's VJP recomputes
+// them, and the buffer holds only the states, dts and checkpoints.
 template <int D, bool kKeep>
 GS_HD int ros23_adjoint_smem_doubles(int K) {
   return K * D + (kKeep ? (K - 1) * (D * D + 5 * D) : 0) + seg_io_doubles<D>(K);
@@ -543,16 +813,18 @@ __device__ __forceinline__ void ros23_adjoint_body(const AdjointArgs& a) {
     for (int q = 1; q < K; ++q) {  // replay steps 0..K-2, keeping their forward quantities
       const double dt = buf.dt(b, q - 1);
       if (dt != 0.0) {
-        RosCore<F> c;
-        double yn[D], s1[D];
-        ros23_core<F>(y, p, dt, c, yn);
         if constexpr (kKeep) {
+          RosCore<F> c;
+          double yn[D], s1[D];
+          ros23_core<F>(y, p, dt, c, yn);
 #pragma unroll
           for (int i = 0; i < D; ++i) s1[i] = y[i] + 0.5 * dt * c.k1[i];
           buf.keep(q - 1, c.W, c.k1, s1, c.k2p);
-        }
 #pragma unroll
-        for (int i = 0; i < D; ++i) y[i] = yn[i];
+          for (int i = 0; i < D; ++i) y[i] = yn[i];
+        } else {
+          ros23_replay_step<F>(y, p, dt);
+        }
       }
 #pragma unroll
       for (int i = 0; i < D; ++i) buf.st(q, i) = y[i];
@@ -563,19 +835,23 @@ __device__ __forceinline__ void ros23_adjoint_body(const AdjointArgs& a) {
         double ys[D];
 #pragma unroll
         for (int i = 0; i < D; ++i) ys[i] = buf.st(q, i);
-        // one VJP call site: the forward quantities come from the replay's kept copy, or
-        // (the segment's last step, or nothing kept) are recomputed here
-        RosCore<F> c;
-        double s1[D];
-        if (kKeep && q < K - 1) {
-          buf.restore(q, c.W, c.k1, s1, c.k2p);
-        } else {
-          double yn[D];
-          ros23_core<F>(ys, p, dt, c, yn);
+        if constexpr (kKeep) {
+          // one VJP call site: the forward quantities come from the replay's kept copy, or
+          // (the segment's last step) are recomputed here
+          RosCore<F> c;
+          double s1[D];
+          if (q < K - 1) {
+            buf.restore(q, c.W, c.k1, s1, c.k2p);
+          } else {
+            double yn[D];
+            ros23_core<F>(ys, p, dt, c, yn);
 #pragma unroll
-          for (int i = 0; i < D; ++i) s1[i] = ys[i] + 0.5 * dt * c.k1[i];
+            for (int i = 0; i < D; ++i) s1[i] = ys[i] + 0.5 * dt * c.k1[i];
+          }
+          ros23_vjp_core<F>(ys, p, dt, c.W, c.k1, s1, c.k2p, lam, gp);
+        } else {
+          ros23_step_vjp<F>(ys, p, dt, lam, gp);
         }
-        ros23_vjp_core<F>(ys, p, dt, c.W, c.k1, s1, c.k2p, lam, gp);
       }
     }
     b ^= 1;

@@ -189,32 +189,56 @@ __device__ __forceinline__ float step_from_sum_f32(float S, float h, const CtrlC
 // of squares S.
 template <int K>
 __device__ __forceinline__ double step_from_sum(double S, double h, const CtrlConsts& c) {
-  double fac;
-  if (S <= c.lo) {
-    fac = Ctrl::FAC_MAX;
-  } else if (S >= c.hi) {
-    fac = Ctrl::FAC_MIN;
-  } else {
-    fac = c.scale * inv_root<K>(S);
-    fac = fac > Ctrl::FAC_MIN ? fac : Ctrl::FAC_MIN;
-    fac = Ctrl::FAC_MAX < fac ? Ctrl::FAC_MAX : fac;
-  }
+  // Selects, not branches: the root is taken of the clamped sum, so every lane runs one path
+  // and the compiler schedules it among the attempt's other work.
+  double fac = c.scale * inv_root<K>(S <= c.lo ? c.lo : (S >= c.hi ? c.hi : S));
+  fac = fac > Ctrl::FAC_MIN ? fac : Ctrl::FAC_MIN;
+  fac = Ctrl::FAC_MAX < fac ? Ctrl::FAC_MAX : fac;
+  fac = S <= c.lo ? Ctrl::FAC_MAX : fac;
+  fac = S >= c.hi ? Ctrl::FAC_MIN : fac;
   return h * fac;
 }
 
+// 1 / x without a branch: the hardware's approximate reciprocal (PTX rcp.approx.ftz.f64, about
+// 2^-20 relative) and one third-order step of the residual series (Householder's method:
+// with e = 1 - x r0, 1 / x = r0 (1 + e + e^2 + ...), truncated below 2^-58), within 2 ulp of
+// the quotient.  Where the approximation is 0, infinite, subnormal or NaN (x infinite, 0 or at
+// the ends of the range) it is the result itself, as the quotient is there.  A division
+// carries a branch to its general case, which the instructions after it cannot be scheduled
+// across; the error norm and W's pivots take one to eight reciprocals per attempt on its
+// dependent chain.
+__device__ __forceinline__ double reciprocal_step(double x, double r0) {
+  const double e = fma(-x, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+__device__ __forceinline__ double reciprocal(double x) {
+  double r0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(x));
+  // exponent field of r0 neither 0 nor 0x7ff (integer pipe)
+  const unsigned ex = ((unsigned)__double2hiint(r0) & 0x7fffffffu) - 0x00100000u;
+  return ex < 0x7fe00000u ? reciprocal_step(x, r0) : r0;
+}
+
 // sum of squares (e_i / sc_i)^2 in numpy's summation order (the reference's np.mean times D).
-// For D <= 4 the D quotients share one division: with P = prod sc_j, e_i / sc_i is taken as
-// e_i * ((prod_{j != i} sc_j) / P), within a few ulp of the quotient (the controller and the
-// accept test read it at that level only where the reference's own Warp and numpy paths
-// already differ), unless P leaves the normal range, where each quotient is divided out.
-template <int D>
+// The quotients are products with reciprocals, within a few ulp of the division (the controller
+// and the accept test read them at that level only where the reference's own Warp and numpy
+// paths already differ).  For 2 <= D <= 4 the components share one: with P = prod sc_j,
+// e_i / sc_i is taken as e_i * ((prod_{j != i} sc_j) / P), unless P leaves the normal range,
+// where each quotient is divided out; larger states and (kShare = false) the latency-bound
+// Rosenbrock23 attempts take one reciprocal per component, which are independent of each other
+// and shorten the attempt's dependent chain.
+//   B200, one division (shared) / shared reciprocal / one per component: forward of Lorenz 2^20,
+//   t = 10: 9.79 / 9.70 / 11.37 ms; Lotka-Volterra 600,001: 583 / 577 / 645 us.  One division
+//   each / one reciprocal each: Lorenz-96 of 8, 50,000 trajectories: 566 / 482 us.  Shared / per
+//   component reciprocal, one Rosenbrock23 attempt of Van der Pol alone: 0.553 / 0.521 us.
+// (The fallback stays a division: a cheap one is predicated, and then runs every time.)
+template <int D, bool kShare = true>
 __device__ __forceinline__ double wrms_sumsq(const double* e, const double* y, const double* yn,
                                              double rtol, double atol) {
   double sc[D], q[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) sc[i] = atol + rtol * fmax(fabs(y[i]), fabs(yn[i]));
-  bool shared = false;
-  if constexpr (D >= 2 && D <= 4) {
+  if constexpr (kShare && D >= 2 && D <= 4) {
     double pre[D], suf[D];  // products of the scales before / after component i
     pre[0] = 1.0;
 #pragma unroll
@@ -224,19 +248,25 @@ __device__ __forceinline__ double wrms_sumsq(const double* e, const double* y, c
     for (int i = D - 2; i >= 0; --i) suf[i] = suf[i + 1] * sc[i + 1];
     const double P = pre[D - 1] * sc[D - 1];
     if (P > 1e-290 && P < 1e290) {
-      shared = true;
-      const double r = 1.0 / P;
+      double r;
+      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(P));
+      r = reciprocal_step(P, r);
 #pragma unroll
       for (int i = 0; i < D; ++i) {
         const double c = e[i] * ((pre[i] * suf[i]) * r);
         q[i] = c * c;
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        const double c = e[i] / sc[i];
+        q[i] = c * c;
+      }
     }
-  }
-  if (!shared) {
+  } else {
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      const double c = e[i] / sc[i];
+      const double c = e[i] * reciprocal(sc[i]);
       q[i] = c * c;
     }
   }

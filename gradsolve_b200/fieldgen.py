@@ -660,6 +660,11 @@ def emit_struct(d: Derived, name: str, code: int) -> str:
     outs += [(f"gp[{j}]", g, "+=") for j, g in enumerate(d.gp) if not _is(g, 0.0)]
     out += _emit_body(outs) + ["    (void)y; (void)p; (void)w; (void)gy; (void)gp;", "  }"]
     if d.stiff:
+        if D <= 8:  # which entries of J are not identically 0 (bit i * D + k)
+            nz = sum(1 << (i * D + k) for i in range(D) for k in range(D)
+                     if not _is(d.J[i][k], 0.0))
+            out += ["  static constexpr GS_HD bool jac_nz(int i, int c) {",
+                    f"    return ({nz:#x}ull >> ({D} * i + c)) & 1;", "  }"]
         out += ["  template <class R>", "  static GS_HD void jac(const R* y, const R* p, R* J) {"]
         out += _emit_body([(f"J[{i * D + k}]", d.J[i][k], "=")
                            for i in range(D) for k in range(D)])
