@@ -19,6 +19,7 @@
 #include "gs_ros23.cuh"
 #include "gs_persistent.cuh"
 #include "gs_saveat.cuh"
+#include "gs_split.cuh"
 #include "gs_tableau.cuh"
 #include "gs_tsit5.cuh"
 
@@ -266,6 +267,20 @@ int persistent_grid(Kern kernel, unsigned block, size_t smem, long long n, unsig
   return GS_OK;
 }
 
+// AUTO's lane refill gives way to one thread per trajectory (float64) where every trajectory of
+// the batch is resident at once: lanes have nothing to refill themselves with then, and the
+// one-thread kernels are shorter per attempt (Van der Pol alone, refilled / one thread: Tsit5
+// 0.684 / 0.525 us, Rosenbrock23 0.689 / 0.521 us).
+template <class Kern>
+int one_wave_schedule(Kern kernel, long long n, int precision, int* sched) {
+  if ((precision & GS_SCHED_MASK) != GS_SCHED_AUTO || *sched == GS_SCHED_STATIC) return GS_OK;
+  unsigned grid = 0;
+  int rc = persistent_grid(kernel, kBlock, 0, n, &grid);
+  if (rc) return rc;
+  if ((long long)grid * kBlock >= n) *sched = GS_SCHED_STATIC;
+  return GS_OK;
+}
+
 int zero_counter(unsigned long long* c, cudaStream_t s) {
   if (!c) return GS_OK;
   cudaError_t e = cudaMemsetAsync(c, 0, sizeof(unsigned long long), s);
@@ -509,6 +524,10 @@ int launch_tsit5_record(const gs::RecordArgs& a_in, cudaStream_t s, bool mixed, 
   if (occ && (mixed || sched != GS_SCHED_STATIC || (!a.rec && !a.ckpt)))
     return fail(GS_ERR_ARG, "GS_OCC applies to the float64 recording forward, one thread per "
                             "trajectory");
+  if (!mixed) {
+    int rc = one_wave_schedule(gs::tsit5_record_kernel<F>, a.n, precision, &sched);
+    if (rc) return rc;
+  }
   if (sched == GS_SCHED_STATIC) {
     if (mixed) {
       gs::tsit5_mixed_record_kernel<F><<<grid_for(a.n), kBlock, 0, s>>>(a);
@@ -636,7 +655,8 @@ int launch_tsit5_adjoint(const gs::AdjointArgs& a, int cap, cudaStream_t s, bool
   }
 }
 template <class F>
-int launch_ros23_record(const gs::RecordArgs& a_in, cudaStream_t s, int sched, int occ) {
+int launch_ros23_record(const gs::RecordArgs& a_in, cudaStream_t s, int sched, int precision) {
+  const int occ = (precision & GS_OCC_MASK) >> GS_OCC_SHIFT;
   gs::RecordArgs a = a_in;
   a.ctrl = gs::make_ctrl_consts(F::D, 6);  // Rosenbrock23: err^(-1/3) = m^(-1/6)
   if (occ && (sched != GS_SCHED_STATIC || (!a.rec && !a.ckpt)))
@@ -656,6 +676,8 @@ int launch_ros23_record(const gs::RecordArgs& a_in, cudaStream_t s, int sched, i
                                 std::to_string(occ) + " blocks per SM is built for D = " +
                                 std::to_string(F::D) + " (gs_occ_choices)");
   }
+  int rc = one_wave_schedule(gs::ros23_record_kernel<F>, a.n, precision, &sched);
+  if (rc) return rc;
   if (sched == GS_SCHED_STATIC) {
     if (!a.rec && !a.ckpt)
       gs::ros23_record_kernel<F, false><<<grid_for(a.n), kBlock, 0, s>>>(a);
@@ -1159,8 +1181,7 @@ int gs_ros23_fwd_record(int field, int precision, long long n, const double* y0,
     GS_ROS23_DISPATCH(field, launch_f32_ros23_record, a, (cudaStream_t)stream)
   }
   GS_ROS23_DISPATCH(field, launch_ros23_record, a, (cudaStream_t)stream,
-                    forward_schedule(precision, t1v, ckpt),
-                    (precision & GS_OCC_MASK) >> GS_OCC_SHIFT)
+                    forward_schedule(precision, t1v, ckpt), precision)
 }
 
 int gs_ros23_replay(int field, int precision, long long n, const double* y0, const double* p,
@@ -1567,19 +1588,83 @@ int launch_fwd_lanes(const gs::RecordArgs& a_in, cudaStream_t s, FwdLanes lanes)
   return cuda_check("record_static_kernel");
 }
 
+// Float64 with a record and checkpoints: the forward alone, then the dense output from them in a
+// pass of its own (gs_split.cuh), so that no lane re-steps while its warp waits.
+template <class F, class M>
+int launch_saveat_states(const gs::RecordArgs& a, cudaStream_t s) {
+  gs::SaveatArgs b{a.n, a.y0, a.p, a.t0, a.rec, a.n_acc, a.ck_every, a.ck_slots, a.ckpt, a.ts,
+                   a.ts_ld, a.K, a.ys, a.yf, nullptr, nullptr, nullptr, nullptr, a.cap};
+  const long long parts = (a.K + gs::kPoints - 1) / gs::kPoints;
+  gs::saveat_states_kernel<F, M><<<grid_for(a.n * parts), kBlock, 0, s>>>(b);
+  return cuda_check("saveat_states_kernel");
+}
+bool states_apart(const gs::RecordArgs& a) { return a.ys && a.rec && a.ckpt; }
+
 template <class F>
-int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed, FwdLanes lanes) {
+int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed, FwdLanes lanes,
+                            int precision) {
   if constexpr (kCoop<F>) {
     return coop_refuse<F>("the dense output (saveat)");
   } else {
-    return mixed ? launch_fwd_lanes<F, gs::LaneTsit5Mixed<F>>(a, s, lanes)
-                 : launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
+    if (mixed) return launch_fwd_lanes<F, gs::LaneTsit5Mixed<F>>(a, s, lanes);
+    if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
+    gs::RecordArgs b = a;
+    b.ys = nullptr;
+    const int sched = lanes == kStatic ? GS_SCHED_STATIC
+                      : lanes == kRefill ? GS_SCHED_REFILL : GS_SCHED_STRIDED;
+    int rc = launch_tsit5_record<F>(b, s, false, sched, precision & GS_SCHED_MASK);
+    return rc ? rc : launch_saveat_states<F, gs::Tsit5F64Step>(a, s);
   }
 }
 
 template <class F>
-int launch_fwd_saveat_ros23(const gs::RecordArgs& a, cudaStream_t s, FwdLanes lanes) {
-  return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
+int launch_fwd_saveat_ros23(const gs::RecordArgs& a, cudaStream_t s, FwdLanes lanes,
+                            int precision) {
+  if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
+  gs::RecordArgs b = a;
+  b.ys = nullptr;
+  const int sched = lanes == kStatic ? GS_SCHED_STATIC
+                    : lanes == kRefill ? GS_SCHED_REFILL : GS_SCHED_STRIDED;
+  int rc = launch_ros23_record<F>(b, s, sched, precision & GS_SCHED_MASK);
+  return rc ? rc : launch_saveat_states<F, gs::Ros23Step>(a, s);
+}
+
+// The reverse pass split over lanes (gs_split.cuh), float64, states of up to kSplitMaxDim.
+template <class F, class S>
+int launch_adjoint_split(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
+                         const long long* order) {
+  if constexpr (F::D > gs::kSplitMaxDim) {
+    return fail(GS_ERR_FIELD, "gs_adjoint_split: built for states of up to " +
+                                  std::to_string(gs::kSplitMaxDim) + " components, not D = " +
+                                  std::to_string(F::D));
+  } else {
+    const int sd = gs::adjoint_smem_doubles<F::D, F::D + 1>(a.ck_every);
+    SegCfg c;
+    int rc;
+    if (a.K > 0) {
+      const long long parts = (a.K + gs::kPoints - 1) / gs::kPoints;
+      gs::saveat_vjp_kernel<F, typename S::Step><<<grid_for(a.n * parts), kBlock, 0, s>>>(a, work);
+      if ((rc = cuda_check("saveat_vjp_kernel"))) return rc;
+      if ((rc = occupancy_cfg(gs::adjoint_split_kernel<F, S, true>, sd, &c))) return rc;
+      gs::adjoint_split_kernel<F, S, true>
+          <<<grid_for_block(a.n * lanes, c.block), c.block, c.smem, s>>>(a, lanes, work, order);
+    } else {
+      if ((rc = occupancy_cfg(gs::adjoint_split_kernel<F, S, false>, sd, &c))) return rc;
+      gs::adjoint_split_kernel<F, S, false>
+          <<<grid_for_block(a.n * lanes, c.block), c.block, c.smem, s>>>(a, lanes, nullptr, order);
+    }
+    return cuda_check("adjoint_split_kernel");
+  }
+}
+template <class F>
+int launch_split_tsit5(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
+                       const long long* order) {
+  return launch_adjoint_split<F, gs::Tsit5Split>(a, s, lanes, work, order);
+}
+template <class F>
+int launch_split_ros23(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
+                       const long long* order) {
+  return launch_adjoint_split<F, gs::Ros23Split>(a, s, lanes, work, order);
 }
 
 int check_saveat(const char* who, long long n, const double* p, const double* rec,
@@ -1653,12 +1738,13 @@ extern "C" int gs_fwd_record_saveat(int method, int field, int precision, long l
   if (method == GS_METHOD_TSIT5) {
     if (prec != GS_PREC_F64 && prec != GS_PREC_MIXED)
       return fail(GS_ERR_PRECISION, std::string(who) + ": unknown precision mode " + std::to_string(prec));
-    GS_TSIT5_DISPATCH(field, launch_fwd_saveat_tsit5, a, s, prec == GS_PREC_MIXED, lanes)
+    GS_TSIT5_DISPATCH(field, launch_fwd_saveat_tsit5, a, s, prec == GS_PREC_MIXED, lanes,
+                      precision)
   }
   if (method == GS_METHOD_ROS23) {
     if (prec != GS_PREC_F64)
       return fail(GS_ERR_PRECISION, std::string(who) + ": Rosenbrock23 runs in float64 only");
-    GS_ROS23_DISPATCH(field, launch_fwd_saveat_ros23, a, s, lanes)
+    GS_ROS23_DISPATCH(field, launch_fwd_saveat_ros23, a, s, lanes, precision)
   }
   return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
 }
@@ -1679,4 +1765,36 @@ extern "C" int gs_adjoint_saveat(int method, int field, int precision, long long
                    const_cast<double*>(ckpt), ts, ts_ld, K, nullptr, nullptr, ysbar, ybar, gy0,
                    gp, cap};
   return saveat_dispatch(method, field, precision, a, stream, true);
+}
+
+extern "C" int gs_adjoint_split(int method, int field, int precision, long long n,
+                                const double* p, const double* rec, const int* n_acc, int cap,
+                                const double* ckpt, int ckpt_every, int lanes, const double* ts,
+                                long long ts_ld, int K, const double* ysbar, double* work,
+                                const double* ybar, double* gy0, double* gp,
+                                const long long* order, void* stream) {
+  const char* who = "gs_adjoint_split";
+  if (precision != GS_PREC_F64)
+    return fail(GS_ERR_PRECISION, std::string(who) + ": float64 without flags only");
+  int rc = check_saveat(who, n, p, rec, n_acc, cap, ckpt, ckpt_every, ts, ts_ld, K);
+  if (rc) return rc;
+  if (lanes < 1 || lanes > 32 || (lanes & (lanes - 1)))
+    return fail(GS_ERR_ARG, std::string(who) + ": lanes must be a power of two up to 32");
+  int D, P;
+  if ((rc = field_dims(field, &D, &P))) return rc;
+  if (n == 0) return GS_OK;
+  if (!ckpt || (K > 0 && (!ysbar || !work)) || (K == 0 && !ybar))
+    return fail(GS_ERR_ARG, std::string(who) + ": ckpt, a cotangent and, with requested times, "
+                                               "work are required");
+  gs::SaveatArgs a{n, nullptr, p, 0.0, rec, n_acc, ckpt_every, gs_ckpt_slots(cap, ckpt_every),
+                   const_cast<double*>(ckpt), ts, ts_ld, K, nullptr, nullptr, ysbar, ybar, gy0,
+                   gp, cap};
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (method == GS_METHOD_TSIT5) {
+    GS_TSIT5_DISPATCH(field, launch_split_tsit5, a, s, lanes, work, order)
+  }
+  if (method == GS_METHOD_ROS23) {
+    GS_ROS23_DISPATCH(field, launch_split_ros23, a, s, lanes, work, order)
+  }
+  return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
 }

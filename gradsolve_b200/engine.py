@@ -590,6 +590,7 @@ def _lanes_flag(method: str, spec: FieldSpec) -> int:
 # the field and is measured once per process on a sample of the caller's trajectories.
 _OCC: dict = {}      # (method, field key) -> GS_OCC blocks per SM of the forward (0: default)
 _OCC_REV: dict = {}  # (method, field key) -> the same for the reverse pass at K = 2
+_OCC_TUNED: dict = {}  # the autotuner's own entries of _OCC_REV (an entry that differs is a pin)
 OCC_MARGIN = 0.01    # another instance replaces the default only when faster by more than 1%
 MIXED = "tsit5/mixed"  # the tables' method key of the Tsit5 float32-stage reverse pass
 _OCC_PASS = {(METHOD_TSIT5, "forward"): 0, (METHOD_TSIT5, "reverse"): 1,
@@ -684,7 +685,7 @@ def autotune_occupancy(spec: FieldSpec, y0: torch.Tensor, p: torch.Tensor, *, t0
     key = (method, spec.key)
     fwd, rev = occ_choices(spec, "forward", method), occ_choices(spec, "reverse", method)
     _OCC[key] = 0
-    _OCC_REV[key] = 0
+    _OCC_REV[key] = _OCC_TUNED[key] = 0
     if len(fwd) < 2:
         return 0, 0
     m = min(y0.shape[0], sample)
@@ -714,6 +715,7 @@ def autotune_occupancy(spec: FieldSpec, y0: torch.Tensor, p: torch.Tensor, *, t0
             adjoint(r, ps, ybar)  # warm
             times[b] = _time_ms(lambda: adjoint(r, ps, ybar), reps)
         _OCC_REV[key] = _pick(times)
+    _OCC_TUNED[key] = _OCC_REV[key]
     return _OCC[key], _OCC_REV[key]
 
 
@@ -1081,6 +1083,65 @@ def _replay_one(r: Record, y0: torch.Tensor, p: torch.Tensor, *, write_ckpt: boo
 
 _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 
+# Lanes per trajectory of the split reverse pass (gs_adjoint_split, csrc/gs_split.cuh), float64
+# states of up to 3 components; 0: one thread per trajectory.  The split costs D (+ 1) step VJPs
+# where one thread takes one, and shortens the chain by the number of lanes: it pays where the
+# batch leaves most of the chip idle, or waits for its longest trajectories.  B200, reverse pass
+# one thread per trajectory / split:
+#   even batches: Lorenz (t = 1, 112 steps) n = 1024 67.6 / 25 us, 4096 67.6 / 39, 16,384 67.8 /
+#   98 (off); Robertson 1024 442 / 45 us;
+#   per-trajectory end times, 64 saved times: stiff Van der Pol 20,011 9.7 / 1.0 ms (16 lanes),
+#   350,000 18.8 / 7.1; Van der Pol 100,003 1.57 / 0.57 ms (4), 700,000 6.06 / 3.27 (1).
+# The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Even
+# Tsit5 batches take it within SPLIT_EVEN_CAP steps of record: over thousands of steps of an
+# expanding flow (Lorenz, t = 70, gradients of 1e20) the two evaluation orders differ by 1e-8.
+SPLIT_MAX_DIM = 3
+SPLIT_EVEN_MAX = 4096
+SPLIT_EVEN_CAP = 4096
+SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without asking for the budget
+
+
+def split_lanes(n: int, dim: int, even: bool, saveat: bool) -> int:
+    if dim > SPLIT_MAX_DIM or (even and not saveat and n > SPLIT_EVEN_MAX) or (
+            not even and not saveat and n > 1 << 17):
+        return 0
+    room = (1 << 16 if even and not saveat else 1 << 19) // max(n, 1)
+    return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
+
+
+def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> bool:
+    if (precision != "float64" or schedule != "auto" or variant != "auto" or
+            not r.y_final.is_cuda or r.spec.dim > SPLIT_MAX_DIM):
+        return False
+    key = (r.method, r.spec.key)  # (a pinned occupancy instance is one thread per trajectory)
+    return key not in _OCC_REV or _OCC_REV[key] == _OCC_TUNED.get(key)
+
+
+def _adjoint_split(r: Record, lanes: int, p, ybar, ts, ysbar, want_y0, want_p, order):
+    L = _lib.lib_for(r.spec)
+    D, dev = r.spec.dim, p.device
+    gy0 = torch.empty((r.n, D), dtype=torch.float64, device=dev) if want_y0 else None
+    gp = torch.empty((r.n, p.shape[1]), dtype=torch.float64, device=dev) if want_p else None
+    ld = K = 0
+    work = None
+    if ts is not None:
+        ts, ld, K = _ts_arg(ts, r.n)
+        work = torch.empty(r.n * K * (D + p.shape[1]), dtype=torch.float64, device=dev)
+    _lib.check(L.gs_adjoint_split(
+        _METHOD_CODE[r.method], r.spec.code, _PREC["float64"], r.n, _ptr(p), _ptr(r.rec),
+        _ptr(r.n_acc), max(r.cap, 1), _ptr(r.ckpt), r.ckpt_every, lanes, _ptr(ts), ld, K,
+        _ptr(ysbar), _ptr(work), _ptr(ybar), _ptr(gy0), _ptr(gp), _ptr(order), _stream()),
+        "gs_adjoint_split", L)
+    return gy0, gp
+
+
+def _lane_order(r: Record, in_batch_order: bool) -> Optional[torch.Tensor]:
+    """The order of a batch-order record's reverse lanes by step count (planned tiers are
+    already ordered), None below ORDER_LANES_MIN."""
+    if not in_batch_order or r.n < ORDER_LANES_MIN:
+        return None
+    return r.lane_order if r.lane_order is not None else prepare_lane_order(r)
+
 
 def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
             want_p: bool = True, precision: str = "float64", schedule: str = "auto",
@@ -1094,8 +1155,17 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
     recomputing kernel's resident threads, else "recompute".  On the float32 route (Tsit5)
     "pairs" runs two trajectories per thread in packed float32x2 arithmetic (built-in
     nonstiff fields), "recompute" one per thread, and "auto" is "pairs" where it is built."""
+    lanes = 0
+    if _split_applies(r, precision, schedule, variant) and (
+            r.uneven or r.method == METHOD_ROS23 or r.cap <= SPLIT_EVEN_CAP):
+        lanes = split_lanes(r.n, r.spec.dim, not r.uneven, False)
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
+    if lanes:
+        res = _over_parts(r, lambda rr, rows: _adjoint_split(
+            rr, lanes, _take(p, rows), _take(ybar, rows).contiguous(), None, None, want_y0,
+            want_p, _lane_order(rr, rows is None)))
+        return _scatter(r, res, 0), _scatter(r, res, 1)
     res = _over_parts(r, lambda rr, rows: _adjoint_one(
         rr, _take(p, rows), _take(ybar, rows), want_y0=want_y0, want_p=want_p,
         precision=precision, schedule=schedule, variant=variant, in_batch_order=rows is None))
@@ -1133,7 +1203,7 @@ def _adjoint_one(r: Record, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: boo
              (_ADJ[variant] if r.method == METHOD_TSIT5 else 0) |
              _occ_rev_flag(r, precision, schedule, variant))
     if in_batch_order and r.n >= ORDER_LANES_MIN and schedule in ("auto", "static"):
-        order = r.lane_order if r.lane_order is not None else prepare_lane_order(r)
+        order = _lane_order(r, True)
         _lib.check(L.gs_adjoint_ordered(_METHOD_CODE[r.method], r.spec.code, flags, r.n, _ptr(p),
                                         _ptr(r.rec), _ptr(r.n_acc), max(r.cap, 1), _ptr(r.ckpt),
                                         r.ckpt_every, _ptr(ybar), _ptr(gy0), _ptr(gp),
@@ -1259,8 +1329,18 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
                    ybar: Optional[torch.Tensor] = None, *, want_y0: bool = True,
                    want_p: bool = True, precision: str = "float64", schedule: str = "auto"):
     """(dL/dy0, dL/dp) for cotangents ysbar = dL/dys (n, K, D) and ybar = dL/dy_final.
-    ``schedule="auto"`` refills lanes from a work counter for an uneven batch (per-trajectory
-    end times), else runs one thread per trajectory."""
+    ``schedule="auto"``, float64, up to 3 components: the split reverse pass; else it refills
+    lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
+    per trajectory for an even one."""
+    if _split_applies(r, precision, schedule):
+        words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
+        if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
+            lanes = split_lanes(r.n, r.spec.dim, not r.uneven, True)
+            f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
+            res = _over_parts(r, lambda rr, rows: _adjoint_split(
+                rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
+                f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None)))
+            return _scatter(r, res, 0), _scatter(r, res, 1)
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
     res = _over_parts(r, lambda rr, rows: _adjoint_saveat_one(

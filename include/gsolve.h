@@ -304,14 +304,14 @@ int gs_replay_saveat(int method, int field, int precision, long long n, const do
 
 /*
  * The adaptive forward with record (gs_tsit5_fwd_record / gs_ros23_fwd_record) that also
- * produces the dense output of gs_replay_saveat at the same time: each requested time is
- * re-stepped from the start of the accepted step that brackets it, as the trajectory is
- * integrated, so the recording point needs no separate replay pass.  ys equals what
- * gs_replay_saveat gives on the recorded mesh to rounding (the same step function, compiled
- * into another kernel).  Schedules: lanes refilled from a work counter (GS_SCHED_REFILL, or
- * AUTO when trajectories have their own end times; needs ckpt), persistent strided lanes
- * (GS_SCHED_STRIDED), one thread per trajectory otherwise (GS_SCHED_STATIC, or AUTO with a
- * shared end time).  No counterpart in the reference,
+ * produces the dense output of gs_replay_saveat at the recording point: each requested time is
+ * re-stepped from the start of the accepted step that brackets it, in float64 with rec and ckpt
+ * by a second kernel from the checkpoints (a thread per few requested times), else as the
+ * trajectory is integrated.  ys equals what gs_replay_saveat gives on the recorded mesh to
+ * rounding (the same step function, compiled into another kernel).  Schedules: lanes refilled
+ * from a work counter (GS_SCHED_REFILL, or AUTO when trajectories have their own end times and
+ * are more than the chip holds at once; needs ckpt), persistent strided lanes
+ * (GS_SCHED_STRIDED), one thread per trajectory otherwise (GS_SCHED_STATIC, or AUTO).  No counterpart in the reference,
  * whose saveat always replays the recorded mesh (gradsolve/warp/warp_replay.py:58-84).
  * method: GS_METHOD_TSIT5 (float64 or mixed) or GS_METHOD_ROS23 (float64).
  */
@@ -335,6 +335,23 @@ int gs_adjoint_saveat(int method, int field, int precision, long long n, const d
                       int ckpt_every, const double* ts, long long ts_ld, int K,
                       const double* ysbar, const double* ybar, double* gy0, double* gp,
                       void* stream);
+
+/*
+ * The reverse pass of gs_tsit5_adjoint / gs_ros23_adjoint (K = 0: ybar required, ts, ysbar and
+ * work NULL) or gs_adjoint_saveat (K > 0) with the steps of each trajectory split over `lanes`
+ * threads (a power of two up to 32): for batches too small to fill the chip with one thread per
+ * trajectory, or whose longest trajectories set the time.  Each lane runs its part's step VJPs
+ * for the D unit cotangents and the parts are composed, D (+ 1) VJPs per step for a chain
+ * `lanes` times shorter.  Float64, states of up to 3 components (GS_ERR_FIELD above).  work: n *
+ * K * (D + P) doubles of scratch.  order: as gs_adjoint_ordered, or NULL.  Gradients agree with
+ * the unsplit passes to rounding and depend on neither ckpt_every nor the rest of the batch.
+ * No counterpart in the reference.
+ */
+int gs_adjoint_split(int method, int field, int precision, long long n, const double* p,
+                     const double* rec, const int* n_acc, int cap, const double* ckpt,
+                     int ckpt_every, int lanes, const double* ts, long long ts_ld, int K,
+                     const double* ysbar, double* work, const double* ybar, double* gy0,
+                     double* gp, const long long* order, void* stream);
 
 /*
  * Record conversion between the reference's padded (n, S) layout (row j = trajectory j's

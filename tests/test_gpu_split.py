@@ -1,0 +1,122 @@
+"""The reverse pass split over lanes and the dense output from the checkpoints (gs_split.cuh)
+against one thread per trajectory: fields of 1 to 3 components, both methods, lanes from 1 to 32,
+trajectories with fewer steps than lanes, none at all, partial last segments, repeated and end
+times.  Two float64 evaluation orders of the same sums: 1e-10 of the row, the bar this
+repository holds the Rosenbrock23 schedules to."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rowrel(a, b):
+    a, b = a.reshape(a.shape[0], -1).cpu().numpy(), b.reshape(b.shape[0], -1).cpu().numpy()
+    return float(np.max(np.abs(a - b).max(1) / np.maximum(np.abs(b).max(1), 1e-12)))
+
+
+def _batch(cuda, field, n, seed=0):
+    rng = np.random.default_rng(seed)
+    y0, p, t1 = {
+        "linear_1": (rng.uniform(0.5, 2.0, (n, 1)), np.zeros((n, 1)), 1.0),
+        "vdp": (rng.uniform(-2, 2, (n, 2)), 10 ** rng.uniform(0.0, 1.2, (n, 1)), 2.0),
+        "lv": (rng.uniform(0.5, 2, (n, 2)), rng.uniform(0.5, 1.5, (n, 4)), 5.0),
+        "lorenz": (rng.uniform(-1, 2, (n, 3)), rng.uniform(20, 30, (n, 1)), 1.0),
+        "lorenz3": (rng.uniform(-1, 2, (n, 3)),
+                    np.stack([rng.uniform(9, 11, n), rng.uniform(2, 3, n),
+                              rng.uniform(20, 30, n)], 1), 1.0),
+        "robertson": (np.tile([1.0, 0.0, 0.0], (n, 1)),
+                      np.array([0.04, 3e7, 1e4]) * 10 ** rng.uniform(-0.5, 0.5, (n, 3)), 10.0),
+    }[field]
+    t1v = t1 * rng.uniform(0.05, 1.0, n)
+    t1v[n // 2] = 0.0  # a trajectory without steps
+    return [torch.tensor(x, device=cuda) for x in (y0, p, t1v)]
+
+
+# (Robertson is stiff: on an explicit method's stability limit the frozen replay itself loses
+# every digit in float64 -- 1e-4 to 1e9 relative against 80-bit arithmetic, split or not)
+CASES = [("tsit5", f) for f in ("linear_1", "vdp", "lv", "lorenz", "lorenz3")] + \
+        [("rosenbrock23", f) for f in ("linear_1", "vdp", "robertson")]
+
+
+@pytest.mark.parametrize("method,field", CASES)
+def test_split_matches_one_thread(gslib, cuda, method, field):
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec = field_spec(field)
+    for n in (1, 3, 37):
+        y0, p, t1v = _batch(cuda, field, n)
+        for K in (1, 3, 64):
+            r = engine.forward_record(method, spec, y0, p, t0=0.0, t1=10.0, t1v=t1v, rtol=1e-6,
+                                      atol=1e-9, checkpoint=K, max_steps=50000, cap0=50000)
+            assert int(r.status.max()) == 0
+            ybar = torch.cos(torch.arange(r.y_final.numel(), device=cuda,
+                                          dtype=torch.float64)).reshape(r.y_final.shape)
+            ref = engine.adjoint(r, p, ybar, schedule="static")
+            back = torch.arange(n - 1, -1, -1, device=cuda)
+            first = {}
+            for lanes in (1, 2, 8, 32):
+                got = engine._adjoint_split(r, lanes, p, ybar, None, None, True, True, None)
+                for a, b in zip(got, ref):
+                    assert rowrel(a, b) <= 1e-10, (n, K, lanes)
+                perm = engine._adjoint_split(r, lanes, p, ybar, None, None, True, True, back)
+                for a, b in zip(got, perm):  # whichever warp takes which trajectory
+                    assert torch.equal(a, b), (n, K, lanes)
+                first[lanes] = got
+            auto = engine.adjoint(r, p, ybar)
+            lanes = engine.split_lanes(n, spec.dim, False, False)
+            if engine._split_applies(r, "float64", "auto"):
+                assert all(torch.equal(a, b) for a, b in zip(auto, first[lanes]))
+
+
+@pytest.mark.parametrize("method,field", CASES)
+def test_split_dense_output(gslib, cuda, method, field):
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec = field_spec(field)
+    n = 37
+    y0, p, t1v = _batch(cuda, field, n, seed=1)
+    row = torch.tensor([0.0, 0.0, 0.01, 0.3, 0.3, 0.77, 0.999, 1.0, 1.0], device=cuda,
+                       dtype=torch.float64)
+    for shared in (False, True):
+        tv = None if shared else t1v
+        t1 = float(t1v.max())
+        ts = t1 * row if shared else t1v[:, None] * row[None, :]
+        for K in (1, 3, 64):
+            kw = dict(t0=0.0, t1=t1, t1v=tv, rtol=1e-6, atol=1e-9, checkpoint=K,
+                      max_steps=50000, cap0=50000)
+            r = engine.forward_record(method, spec, y0, p, saveat_ts=ts, **kw)
+            yf, ys = engine.replay_saveat(r, y0, p, ts, write_ckpt=False)
+            assert rowrel(r.ys, ys) <= 1e-10
+            assert torch.equal(r.ys[:, -1], r.y_final) and torch.equal(r.ys[:, 0], y0)
+            ysbar = torch.sin(1.0 + torch.arange(ys.numel(), device=cuda,
+                                                 dtype=torch.float64)).reshape(ys.shape)
+            ybar = torch.ones_like(yf)
+            for yb in (None, ybar):
+                ref = engine.adjoint_saveat(r, p, ts, ysbar, yb, schedule="static")
+                for lanes in (1, 4, 32):
+                    got = engine._adjoint_split(r, lanes, p, yb, ts, ysbar, True, True, None)
+                    for a, b in zip(got, ref):
+                        assert rowrel(a, b) <= 1e-10, (shared, K, lanes)
+
+
+def test_split_refuses(gslib, cuda):
+    from gradsolve_b200 import engine
+    from gradsolve_b200._lib import GsolveError
+    from gradsolve_b200.fields import field_spec
+    y0, p, t1v = _batch(cuda, "lorenz", 5)
+    r = engine.forward_record("tsit5", field_spec("lorenz"), y0, p, t0=0.0, t1=1.0, rtol=1e-6,
+                              atol=1e-9, checkpoint=2)
+    with pytest.raises(GsolveError, match="power of two"):
+        engine._adjoint_split(r, 3, p, r.y_final, None, None, True, True, None)
+    with pytest.raises(GsolveError, match="cotangent"):
+        engine._adjoint_split(r, 2, p, None, None, None, True, True, None)
+    spec = field_spec("hires")
+    y8 = torch.rand(4, 8, device=cuda, dtype=torch.float64)
+    p8 = torch.zeros(4, 1, device=cuda, dtype=torch.float64)
+    r8 = engine.forward_record("tsit5", spec, y8, p8, t0=0.0, t1=0.1, rtol=1e-6, atol=1e-9,
+                               checkpoint=2)
+    with pytest.raises(GsolveError, match="up to 3 components"):
+        engine._adjoint_split(r8, 2, p8, r8.y_final, None, None, True, True, None)
