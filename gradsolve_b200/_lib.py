@@ -70,6 +70,7 @@ _SIGS = {
     "gs_adjoint_saveat": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p,
                                   c_int, c_void_p, c_int, c_void_p, c_ll, c_int, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_void_p]),
+    "gs_lane_order": (c_int, [c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "gs_adjoint_split": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_int,
                                  c_void_p, c_int, c_int, c_void_p, c_ll, c_int, c_void_p,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),

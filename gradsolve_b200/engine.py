@@ -151,6 +151,7 @@ def first_capacity(n: int, dim: int, max_steps: int, ckpt_every: int, precision:
 # process on a sample of the caller's own trajectories and cached.
 _TUNED: dict = {}
 TUNE_CANDIDATES = (2, 3, 4, 6, 8, 12, 16)
+TUNE_MIXED, TUNE_MARGIN_MIXED = 4, 0.04  # (Lotka-Volterra 2^18: K = 2, 3, 4 within 3%, 8 4% off)
 _IN_TUNER = [0]  # nonzero while an autotuner runs its own forwards (no nested tuning)
 
 
@@ -193,7 +194,7 @@ def autotune_ckpt_every(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch
         candidates = TUNE_CANDIDATES_F32 if precision == "float32" else TUNE_CANDIDATES
     budget = _checkpoint_budget()
     row = 4 * ckpt_width_f32(spec.dim) if precision == "float32" else 8 * ckpt_width(spec.dim)
-    best, best_ms = None, float("inf")
+    times = {}
     for K in candidates:
         if (DEFAULT_CAP0 // K + 2) * m * row > budget and K != candidates[-1]:
             continue  # this interval's checkpoints would not fit beside the caller's data
@@ -216,8 +217,13 @@ def autotune_ckpt_every(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch
             e1.record()
             e1.synchronize()
             ms = min(ms, e0.elapsed_time(e1))
-        if ms < best_ms:
-            best, best_ms = K, ms
+        times[K] = ms
+    best = min(times, key=times.get)
+    if precision == "mixed" and times.get(TUNE_MIXED, float("inf")) <= \
+            times[best] * (1.0 + TUNE_MARGIN_MIXED):
+        # the float32-stage gradient's rounding depends on the interval (on which steps' stages
+        # are kept), so near-equal intervals must not swap places from run to run
+        best = TUNE_MIXED
     _TUNED[(method, spec.key, precision)] = best
     return best
 
@@ -329,9 +335,10 @@ class RecordSet:
         """For each part, the rows whose final tier it is, longest first (by this record's
         step counts): lanes refilled from a work counter then take the long trajectories
         first, and the short ones fill in around them instead of the long ones ending last."""
-        if len(self.parts) == 1 and self.parts[0][0] is None:  # one tier: no host sync
-            cost = (self.n_acc + self.n_rej).to(torch.int64)
-            return [torch.argsort(cost, descending=True, stable=True)]
+        if len(self.parts) == 1:  # one tier, whatever its rows' order: no host sync
+            if self.uneven and self.n > WINDOW_UNEVEN:  # (the longest first over the batch)
+                return [torch.argsort(self.n_acc + self.n_rej, descending=True, stable=True)]
+            return [_window_order(self.n_acc, self.n_rej, WINDOW_UNEVEN)]
         owner = torch.zeros(self.n, dtype=torch.int64, device=self.y_final.device)
         for k, (rows, _r) in enumerate(self.parts):
             if rows is None:
@@ -1172,20 +1179,37 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
     return _scatter(r, res, 0), _scatter(r, res, 1)
 
 
+def _window_order(a: torch.Tensor, b: Optional[torch.Tensor], window: int) -> torch.Tensor:
+    """gs_lane_order of int32 device counts (their stable descending order, off the GPU)."""
+    if not a.is_cuda:
+        return torch.argsort(a if b is None else a + b, descending=True, stable=True)
+    order = torch.empty(a.shape[0], dtype=torch.int64, device=a.device)
+    L = _lib.lib()
+    _lib.check(L.gs_lane_order(a.shape[0], _ptr(a), _ptr(b), window, _ptr(order), _stream()),
+               "gs_lane_order", L)
+    return order
+
+
 def prepare_lane_order(r) -> Optional[torch.Tensor]:
     """Queue the sort that orders a batch-order record's reverse lanes by step count (longest
-    first) on the current stream, so it runs while the host prepares the cotangent; the
-    reverse pass picks it up.  Planned records (already ordered by cost) need none."""
+    first) on the current stream; the reverse pass picks it up.  Planned records (already ordered
+    by cost) need none."""
     if isinstance(r, Record) and r.n >= ORDER_LANES_MIN:
-        r.lane_order = torch.argsort(r.n_acc, descending=True, stable=True)
+        r.lane_order = _window_order(r.n_acc, None, WINDOW_UNEVEN if r.uneven else WINDOW_EVEN)
         return r.lane_order
     return None
 
 
+# Trajectories per window of gs_lane_order: small ones keep a warp's checkpoint rows together; the
+# split reverse pass of an uneven batch, whose lanes work at different steps anyway, orders more
+# trajectories, so that its longest ones do not start last.
+WINDOW_EVEN = 512
+WINDOW_UNEVEN = 4096
+
+
 # A record in batch order (a fresh forward; a planned tier is already ordered by cost) runs its
 # reverse pass with the lanes ordered by step count, longest first, from this many
-# trajectories up (the sort costs ~0.1 ms at 2^20 and saves the idle lanes of warps whose
-# trajectories' step counts differ).
+# trajectories up (it saves the idle lanes of warps whose trajectories' step counts differ).
 ORDER_LANES_MIN = 1 << 12
 
 

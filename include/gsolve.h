@@ -376,6 +376,15 @@ int gs_move_rows(int scatter, int elem_bytes, const void* src, const long long* 
                  long long rows, int width, long long limit, void* dst,
                  unsigned long long* bad, void* stream);
 
+/*
+ * An order for gs_adjoint_ordered, gs_adjoint_split and the host's plans: within each window of
+ * `window` (512 or 4096) consecutive trajectories, by a[j] + b[j] (b may be NULL), largest first
+ * and equal ones in batch order.  order: n int64 on the device, a permutation of [0, n).  No
+ * counterpart in the reference.
+ */
+int gs_lane_order(long long n, const int* a, const int* b, int window, long long* order,
+                  void* stream);
+
 /* Size of the library's own device scratch used by gs_tsit5_vjp_static: 64 MiB, held by
  * every GPU that loads libgsolve.so until the process exits.  Only libgsolve.so carries it:
  * the libraries built for generated fields (gradsolve_b200/fieldgen.py) export
