@@ -947,46 +947,74 @@ __global__ void move_rows_kernel(const T* src, const long long* idx, long long r
   }
 }
 
-// Lanes ordered by step count within windows of W consecutive trajectories, longest first (equal
-// counts in batch order): a bitonic sort of (count, index) keys in shared memory, one block per
-// window, W / T keys per thread.  A sort of the whole batch spreads a warp's trajectories over the
+// Lanes ordered by step count within windows of T * E consecutive trajectories, longest first
+// (equal counts in batch order): a bitonic sort of (count, index) keys, E per thread, one block per
+// window; strides within a thread and within a warp run in registers and shuffles, wider ones
+// through shared memory.  A sort of the whole batch spreads a warp's trajectories over the
 // record, and their checkpoint rows and dt sectors then come from DRAM one by one: reverse pass of
 // Lorenz 2^20 (t = 10) 12.8 ms in windows of 512, 13.6 of 1024, 15.0 over the batch, 13.0 in
 // batch order; Lotka-Volterra 600,001 (counts spread 1:3) 769 / 753 / 722 / 1073 us.  And it is
-// one launch of 5 us where the sort of the batch took a dozen and 70-120 us.
-template <int W, int T>
+// one launch where the sort of the batch took a dozen and 70-120 us.
+template <int T, int E>
 __global__ void __launch_bounds__(T) lane_order_kernel(long long n, const int* a, const int* b,
                                                        long long* order) {
-  __shared__ unsigned long long key[W];
+  constexpr int W = T * E;
+  constexpr unsigned kMost = (1u << 20) - 1;  // counts are compared up to here
+  static_assert(W <= 4096, "20 bits of count and 12 of index");
+  __shared__ unsigned sh[W];
+  const int tid = threadIdx.x;
   const long long base = (long long)blockIdx.x * W;
-  for (int i = threadIdx.x; i < W; i += T) {
-    const long long j = base + i;
-    // ascending keys: the complement of the count, then the index; past the batch last
-    unsigned long long k = ~0ull;
-    if (j < n) {
-      const long long c = (long long)a[j] + (b ? b[j] : 0);
-      k = ((unsigned long long)(0x7fffffffll - (c < 0 ? 0 : c > 0x7ffffffell ? 0x7ffffffell : c))
-           << 32) | (unsigned)i;
+  unsigned key[E];  // ascending: the count's complement, then the index; past the batch last
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    key[e] = ~0u;
+    if (base + i < n) {
+      const long long c = (long long)a[base + i] + (b ? b[base + i] : 0);
+      key[e] = (((c < 0 ? kMost : c > (long long)kMost - 1 ? 1u : kMost - (unsigned)c) << 12) |
+                (unsigned)i);
     }
-    key[i] = k;
   }
+#pragma unroll
   for (int size = 2; size <= W; size <<= 1) {
+#pragma unroll
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < W / 2; i += T) {
-        const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-        const bool up = (lo & size) == 0;
-        const unsigned long long x = key[lo], y = key[hi];
-        if ((x > y) == up) {
-          key[lo] = y;
-          key[hi] = x;
+      if (stride < E) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int o = e ^ stride;
+          if (o > e) {
+            const bool up = ((tid * E + e) & size) == 0;
+            const unsigned x = key[e], y = key[o];
+            const unsigned lo = x < y ? x : y, hi = x < y ? y : x;
+            key[e] = up ? lo : hi;
+            key[o] = up ? hi : lo;
+          }
+        }
+      } else {
+        const int far = stride / E;  // the partner thread is tid ^ far
+        if (far >= 32) {
+          __syncthreads();
+#pragma unroll
+          for (int e = 0; e < E; ++e) sh[e * T + tid] = key[e];
+          __syncthreads();
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const unsigned other =
+              far >= 32 ? sh[e * T + (tid ^ far)] : __shfl_xor_sync(0xffffffffu, key[e], far & 31);
+          const bool up = ((tid * E + e) & size) == 0, low = (tid & far) == 0;
+          const bool least = up == low;
+          key[e] = (key[e] < other) == least ? key[e] : other;
         }
       }
     }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < W && base + i < n; i += T)
-    order[base + i] = base + (long long)(unsigned)key[i];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    if (base + i < n) order[base + i] = base + (long long)(key[e] & 4095u);
+  }
 }
 
 int check_record_args(const char* who, long long n, const double* y0, const double* p,
@@ -1355,9 +1383,9 @@ int gs_lane_order(long long n, const int* a, const int* b, int window, long long
   const unsigned grid = (unsigned)((n + window - 1) / window);
   const cudaStream_t s = (cudaStream_t)stream;
   if (window == 512)
-    lane_order_kernel<512, 256><<<grid, 256, 0, s>>>(n, a, b, order);
+    lane_order_kernel<512, 1><<<grid, 512, 0, s>>>(n, a, b, order);
   else
-    lane_order_kernel<4096, 1024><<<grid, 1024, 0, s>>>(n, a, b, order);
+    lane_order_kernel<1024, 4><<<grid, 1024, 0, s>>>(n, a, b, order);
   return cuda_check("lane_order_kernel");
 }
 

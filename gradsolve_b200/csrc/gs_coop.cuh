@@ -235,8 +235,9 @@ __global__ void __launch_bounds__(128) tsit5_coop_replay_kernel(const ReplayArgs
   const bool ck_on = a.ckpt != nullptr;
   if (ck_on) coop_store_ckpt<F, G>(a.ckpt, a.n, j, 0, y, t);
   int ck_cnt = 0, ck_slot = 0;
+  DtStream dts(a.rec, a.n, j, na);
   for (int s = 0; s < na; ++s) {
-    const double dt = load_rec(a.rec, a.n, j, s);
+    const double dt = dts.take(s);
     tsit5_replay_step<L>(y, p, dt);
     t = t + dt;
     if (ck_on && ++ck_cnt == a.ck_every) {

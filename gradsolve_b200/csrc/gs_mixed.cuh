@@ -208,7 +208,7 @@ __device__ __forceinline__ void mixed_vjp_core(const Src& src, const float* pf, 
   }
   src.template get<6>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = 0.0f;
+  for (int i = 0; i < D; ++i) sb[i] = -0.0f;
   F::vjp(st, pf, kb6, sb, gpf);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
@@ -219,7 +219,7 @@ __device__ __forceinline__ void mixed_vjp_core(const Src& src, const float* pf, 
   }
   src.template get<5>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = 0.0f;
+  for (int i = 0; i < D; ++i) sb[i] = -0.0f;
   F::vjp(st, pf, kb5, sb, gpf);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
@@ -229,7 +229,7 @@ __device__ __forceinline__ void mixed_vjp_core(const Src& src, const float* pf, 
   }
   src.template get<4>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = 0.0f;
+  for (int i = 0; i < D; ++i) sb[i] = -0.0f;
   F::vjp(st, pf, kb4, sb, gpf);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
@@ -239,7 +239,7 @@ __device__ __forceinline__ void mixed_vjp_core(const Src& src, const float* pf, 
   }
   src.template get<3>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = 0.0f;
+  for (int i = 0; i < D; ++i) sb[i] = -0.0f;
   F::vjp(st, pf, kb3, sb, gpf);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
@@ -249,7 +249,7 @@ __device__ __forceinline__ void mixed_vjp_core(const Src& src, const float* pf, 
   }
   src.template get<2>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = 0.0f;
+  for (int i = 0; i < D; ++i) sb[i] = -0.0f;
   F::vjp(st, pf, kb2, sb, gpf);
 #pragma unroll
   for (int i = 0; i < D; ++i) {

@@ -455,8 +455,10 @@ __device__ __forceinline__ bool ros23_trial_as(const double* y, const double* p,
   for (int i = 0; i < D; ++i)
     r3[i] = F2[i] - Ros23::E32 * (rc.k2[i] - rc.F1[i]) - 2.0 * (rc.k1[i] - rc.F0[i]);
   w_solve<F, kSparse, false>(rc.W, r3, k3);
+  // (h / 6 as a product, within an ulp: a division by a constant is a division in full)
+  const double h6 = h * (1.0 / 6.0);
 #pragma unroll
-  for (int i = 0; i < D; ++i) ev[i] = (h / 6.0) * (rc.k1[i] - 2.0 * rc.k2[i] + k3[i]);
+  for (int i = 0; i < D; ++i) ev[i] = h6 * (rc.k1[i] - 2.0 * rc.k2[i] + k3[i]);
   return ok;
 }
 
@@ -521,14 +523,14 @@ __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, con
     yb[i] = lam[i];
     k2b[i] = dt * lam[i];
     k1b[i] = k2b[i];
-    s1b[i] = R(0.0);
+    s1b[i] = R(-0.0);  // (the identity of addition, +0 is not)
   }
   w_solve<F, kSparse, true>(W, k2b, r2b);
   const R scale = R(Ros23::D) * dt;  // G = -d dt Wbar, Wbar = -(r2b k2p^T + r1b k1^T)
 #pragma unroll
   for (int i = 0; i < D; ++i) {
 #pragma unroll
-    for (int c = 0; c < D; ++c) G[i * D + c] = scale * (r2b[i] * k2p[c]);
+    for (int c = 0; c < D; ++c) G[i * D + c] = r2b[i] * k2p[c];
     k1b[i] -= r2b[i];
   }
   F::vjp(s1, p, r2b, s1b, gp);
@@ -541,7 +543,7 @@ __device__ __forceinline__ void ros23_vjp_core(const R* y, const R* p, R dt, con
 #pragma unroll
   for (int i = 0; i < D; ++i)
 #pragma unroll
-    for (int c = 0; c < D; ++c) G[i * D + c] += scale * (r1b[i] * k1[c]);
+    for (int c = 0; c < D; ++c) G[i * D + c] = scale * (G[i * D + c] + r1b[i] * k1[c]);
   F::vjp(y, p, r1b, yb, gp);
   F::jac_contract_grad(y, p, G, yb, gp);
 #pragma unroll
@@ -711,8 +713,9 @@ __global__ void __launch_bounds__(128) ros23_replay_kernel(const ReplayArgs a) {
   const bool ck_on = a.ckpt != nullptr;
   if (ck_on) store_ckpt<D>(a.ckpt, a.n, j, 0, y, t);
   int ck_cnt = 0, ck_slot = 0;
+  DtStream dts(a.rec, a.n, j, na);
   for (int s = 0; s < na; ++s) {
-    const double dt = load_rec(a.rec, a.n, j, s);
+    const double dt = dts.take(s);
     ros23_replay_step<F>(y, p, dt);
     t = t + dt;
     if (ck_on && ++ck_cnt == a.ck_every) {

@@ -121,8 +121,9 @@ __global__ void __launch_bounds__(128) replay_saveat_kernel(const SaveatArgs a) 
   const bool ck_on = a.ckpt != nullptr;
   if (ck_on) store_ckpt<D>(a.ckpt, a.n, j, 0, y, t);
   int ck_cnt = 0, ck_slot = 0;
+  DtStream dts(a.rec, a.n, j, na);
   for (int s = 0; s < na; ++s) {
-    const double dt = load_rec(a.rec, a.n, j, s);
+    const double dt = dts.take(s);
     if (dt > 0.0) {
       const double tn = t + dt;
       while (kk < a.K && ts[kk] <= tn) {  // bracketed by this step: re-step to ts

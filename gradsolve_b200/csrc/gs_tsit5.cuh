@@ -190,10 +190,11 @@ __device__ __forceinline__ float step_from_sum_f32(float S, float h, const CtrlC
 template <int K>
 __device__ __forceinline__ double step_from_sum(double S, double h, const CtrlConsts& c) {
   // Selects, not branches: the root is taken of the clamped sum, so every lane runs one path
-  // and the compiler schedules it among the attempt's other work.
+  // and the compiler schedules it among the attempt's other work.  Clipping the factor again
+  // is two comparisons on the attempt's chain for an ulp (a Van der Pol Rosenbrock23 attempt 0.478
+  // / 0.462 us, forward of Lotka-Volterra 600,001 577 / 562 us).
   double fac = c.scale * inv_root<K>(S <= c.lo ? c.lo : (S >= c.hi ? c.hi : S));
-  fac = fac > Ctrl::FAC_MIN ? fac : Ctrl::FAC_MIN;
-  fac = Ctrl::FAC_MAX < fac ? Ctrl::FAC_MAX : fac;
+  // (of a sum inside the clips' range the factor is inside them too, within an ulp)
   fac = S <= c.lo ? Ctrl::FAC_MAX : fac;
   fac = S >= c.hi ? Ctrl::FAC_MIN : fac;
   return h * fac;
@@ -383,6 +384,15 @@ __device__ __forceinline__ void tsit5_stage_states(const R* y, const R* p, R dt,
   }
 }
 
+// c + a b, in float64 fused explicitly: of the two products of B g + A u the same one in every
+// instance of a kernel.
+template <class R, class B>
+__device__ __forceinline__ R madd(R a, B b, R c) {
+  c += a * b;
+  return c;
+}
+__device__ __forceinline__ double madd(double a, double b, double c) { return fma(a, b, c); }
+
 // Reverse of one replay step at (y, dt) given its stage inputs (Src::get<M> yields s_M):
 // lam <- (dy'/dy)^T lam, gp += (dy'/dp)^T lam.  Stage 7 carries weight B7 == 0, so its
 // cotangent is exactly zero and it is skipped.
@@ -390,88 +400,91 @@ template <class F, class Src, class R = double>
 __device__ __forceinline__ void tsit5_vjp_core(const R* y, const Src& src, const R* p, R dt,
                                                R* lam, R* gp) {
   constexpr int D = F::D;
-  using T = Tsit5;
+#define GS_C(x) vjp_coef<R>(Tsit5::x, kTsit5Table.x)
   R st[D];
   R g[D], kb1[D], kb2[D], kb3[D], kb4[D], kb5[D], kb6[D], sb[D], yb[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     g[i] = dt * lam[i];
     yb[i] = lam[i];
-    kb1[i] = R(T::B1) * g[i];
-    kb2[i] = R(T::B2) * g[i];
-    kb3[i] = R(T::B3) * g[i];
-    kb4[i] = R(T::B4) * g[i];
-    kb5[i] = R(T::B5) * g[i];
-    kb6[i] = R(T::B6) * g[i];
+    kb1[i] = GS_C(B1) * g[i];
+    kb2[i] = GS_C(B2) * g[i];
+    kb3[i] = GS_C(B3) * g[i];
+    kb4[i] = GS_C(B4) * g[i];
+    kb5[i] = GS_C(B5) * g[i];
+    kb6[i] = GS_C(B6) * g[i];
   }
+  // (sb starts at -0, the identity of addition: from +0 the field's `gy += ...` is an addition
+  // that cannot be left out, 5 D of them per step)
   // stage 6
   src.template get<6>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = R(0.0);
+  for (int i = 0; i < D; ++i) sb[i] = R(-0.0);
   F::vjp(st, p, kb6, sb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     yb[i] += sb[i];
     const R u = dt * sb[i];
-    kb1[i] += R(T::A61) * u;
-    kb2[i] += R(T::A62) * u;
-    kb3[i] += R(T::A63) * u;
-    kb4[i] += R(T::A64) * u;
-    kb5[i] += R(T::A65) * u;
+    kb1[i] = madd(GS_C(A61), u, kb1[i]);
+    kb2[i] = madd(GS_C(A62), u, kb2[i]);
+    kb3[i] = madd(GS_C(A63), u, kb3[i]);
+    kb4[i] = madd(GS_C(A64), u, kb4[i]);
+    kb5[i] = madd(GS_C(A65), u, kb5[i]);
   }
   // stage 5
   src.template get<5>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = R(0.0);
+  for (int i = 0; i < D; ++i) sb[i] = R(-0.0);
   F::vjp(st, p, kb5, sb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     yb[i] += sb[i];
     const R u = dt * sb[i];
-    kb1[i] += R(T::A51) * u;
-    kb2[i] += R(T::A52) * u;
-    kb3[i] += R(T::A53) * u;
-    kb4[i] += R(T::A54) * u;
+    kb1[i] = madd(GS_C(A51), u, kb1[i]);
+    kb2[i] = madd(GS_C(A52), u, kb2[i]);
+    kb3[i] = madd(GS_C(A53), u, kb3[i]);
+    kb4[i] = madd(GS_C(A54), u, kb4[i]);
   }
   // stage 4
   src.template get<4>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = R(0.0);
+  for (int i = 0; i < D; ++i) sb[i] = R(-0.0);
   F::vjp(st, p, kb4, sb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     yb[i] += sb[i];
     const R u = dt * sb[i];
-    kb1[i] += R(T::A41) * u;
-    kb2[i] += R(T::A42) * u;
-    kb3[i] += R(T::A43) * u;
+    kb1[i] = madd(GS_C(A41), u, kb1[i]);
+    kb2[i] = madd(GS_C(A42), u, kb2[i]);
+    kb3[i] = madd(GS_C(A43), u, kb3[i]);
   }
   // stage 3
   src.template get<3>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = R(0.0);
+  for (int i = 0; i < D; ++i) sb[i] = R(-0.0);
   F::vjp(st, p, kb3, sb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     yb[i] += sb[i];
     const R u = dt * sb[i];
-    kb1[i] += R(T::A31) * u;
-    kb2[i] += R(T::A32) * u;
+    kb1[i] = madd(GS_C(A31), u, kb1[i]);
+    kb2[i] = madd(GS_C(A32), u, kb2[i]);
   }
   // stage 2
   src.template get<2>(st);
 #pragma unroll
-  for (int i = 0; i < D; ++i) sb[i] = R(0.0);
+  for (int i = 0; i < D; ++i) sb[i] = R(-0.0);
   F::vjp(st, p, kb2, sb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     yb[i] += sb[i];
-    kb1[i] += R(T::A21) * (dt * sb[i]);
+    kb1[i] = madd(GS_C(A21), dt * sb[i], kb1[i]);
   }
   // stage 1 (s1 = y)
   F::vjp(y, p, kb1, yb, gp);
 #pragma unroll
   for (int i = 0; i < D; ++i) lam[i] = yb[i];
+#undef GS_C
 }
 
 // Reverse of one replay step, recomputing its stages from y.
@@ -590,6 +603,43 @@ __device__ __forceinline__ void store_rec_chunk(double* rec, long long n, long l
   dst[0] = make_double2(a, b);
   dst[1] = make_double2(c, d);
 }
+
+// A trajectory's dts in order, one record sector (4 steps, 32 bytes) ahead of the step that is
+// integrated: the replay's chain then waits on no load (Lorenz alone 0.34 us per step with a
+// load in each).
+struct DtStream {
+  const double2* next;
+  size_t stride;  // double2's from one of the trajectory's sectors to the next
+  int left;       // sectors not yet loaded
+  double2 a0, a1, b0, b1;  // the current sector and the one after it
+  __device__ __forceinline__ DtStream(const double* rec, long long n, long long j, int na)
+      : next(reinterpret_cast<const double2*>(rec) + 2 * (size_t)j), stride(2 * (size_t)n),
+        left((na + 3) >> 2) {
+    a0 = a1 = b0 = b1 = make_double2(0.0, 0.0);
+    load();
+    a0 = b0;
+    a1 = b1;
+    load();
+  }
+  __device__ __forceinline__ void load() {
+    if (left > 0) {
+      b0 = __ldg(next);
+      b1 = __ldg(next + 1);
+      next += stride;
+      --left;
+    }
+  }
+  // dt of step s (called for s = 0, 1, 2, ... in turn)
+  __device__ __forceinline__ double take(int s) {
+    const double dt = (s & 2) ? ((s & 1) ? a1.y : a1.x) : ((s & 1) ? a0.y : a0.x);
+    if ((s & 3) == 3) {
+      a0 = b0;
+      a1 = b1;
+      load();
+    }
+    return dt;
+  }
+};
 
 __device__ __forceinline__ double load_rec(const double* rec, long long n, long long j,
                                            long long s) {
@@ -724,8 +774,9 @@ __global__ void __launch_bounds__(128) tsit5_replay_kernel(const ReplayArgs a) {
   const bool ck_on = a.ckpt != nullptr;
   if (ck_on) store_ckpt<D>(a.ckpt, a.n, j, 0, y, t);
   int ck_cnt = 0, ck_slot = 0;
+  DtStream dts(a.rec, a.n, j, na);
   for (int s = 0; s < na; ++s) {
-    const double dt = load_rec(a.rec, a.n, j, s);
+    const double dt = dts.take(s);
     tsit5_replay_step<F>(y, p, dt);
     t = t + dt;
     if (ck_on && ++ck_cnt == a.ck_every) {

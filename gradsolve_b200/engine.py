@@ -629,6 +629,8 @@ def set_occupancy(spec: FieldSpec, blocks: Optional[int], pass_: str = "forward"
     """Pin the occupancy instance of a field's forward or reverse pass (None: back to
     autotuning)."""
     table = _OCC if pass_ == "forward" else _OCC_REV
+    if pass_ == "reverse":
+        _OCC_TUNED.pop((method, spec.key), None)  # what the table holds from here on is a pin
     if blocks is None:
         table.pop((method, spec.key), None)
         return

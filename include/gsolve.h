@@ -378,8 +378,8 @@ int gs_move_rows(int scatter, int elem_bytes, const void* src, const long long* 
 
 /*
  * An order for gs_adjoint_ordered, gs_adjoint_split and the host's plans: within each window of
- * `window` (512 or 4096) consecutive trajectories, by a[j] + b[j] (b may be NULL), largest first
- * and equal ones in batch order.  order: n int64 on the device, a permutation of [0, n).  No
+ * `window` (512 or 4096) consecutive trajectories, by a[j] + b[j] (b may be NULL; counts compared
+ * up to 2^20 - 2), largest first and equal ones in batch order.  order: n int64 on the device, a permutation of [0, n).  No
  * counterpart in the reference.
  */
 int gs_lane_order(long long n, const int* a, const int* b, int window, long long* order,
