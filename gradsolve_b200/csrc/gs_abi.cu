@@ -16,6 +16,7 @@
 #include "gs_f32.cuh"
 #include "gs_fields.cuh"
 #include "gs_mixed.cuh"
+#include "gs_paired.cuh"
 #include "gs_ros23.cuh"
 #include "gs_persistent.cuh"
 #include "gs_saveat.cuh"
@@ -1742,14 +1743,38 @@ int launch_adjoint_split(const gs::SaveatArgs& a, cudaStream_t s, int lanes, dou
     return cuda_check("adjoint_split_kernel");
   }
 }
+// ... or run by two warps per 32 trajectories (gs_paired.cuh), states of up to 8 components.
+template <class F, class S>
+int launch_adjoint_paired(const gs::SaveatArgs& a, cudaStream_t s, const long long* order) {
+  const int sd = gs::paired_smem_doubles<F, S>(a.ck_every);
+  const size_t smem = (size_t)sd * 64 * sizeof(double);
+  if (smem > kSegBudget)
+    return fail(GS_ERR_ARG, "gs_adjoint_split: two warps' segments of K = " +
+                                std::to_string(a.ck_every) + " do not fit shared memory");
+  int rc;
+  if ((rc = allow_smem(gs::adjoint_paired_kernel<F, S>, smem))) return rc;
+  gs::AdjointArgs b{a.n, a.p, a.rec, a.n_acc, a.ckpt, a.ck_every, a.ybar, a.gy0, a.gp, a.cap,
+                    order};
+  gs::adjoint_paired_kernel<F, S><<<(unsigned)((a.n + 31) / 32), 64, smem, s>>>(b);
+  return cuda_check("adjoint_paired_kernel");
+}
+
 template <class F>
 int launch_split_tsit5(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
                        const long long* order) {
+  if (lanes == 0) {
+    if constexpr (F::D <= 8) return launch_adjoint_paired<F, gs::Tsit5Pair<F>>(a, s, order);
+    return fail(GS_ERR_FIELD, "gs_adjoint_split: two warps are built for up to 8 components");
+  }
   return launch_adjoint_split<F, gs::Tsit5Split>(a, s, lanes, work, order);
 }
 template <class F>
 int launch_split_ros23(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
                        const long long* order) {
+  if (lanes == 0) {
+    if constexpr (F::D <= 8) return launch_adjoint_paired<F, gs::Ros23Pair<F>>(a, s, order);
+    return fail(GS_ERR_FIELD, "gs_adjoint_split: two warps are built for up to 8 components");
+  }
   return launch_adjoint_split<F, gs::Ros23Split>(a, s, lanes, work, order);
 }
 
@@ -1864,8 +1889,9 @@ extern "C" int gs_adjoint_split(int method, int field, int precision, long long 
     return fail(GS_ERR_PRECISION, std::string(who) + ": float64 without flags only");
   int rc = check_saveat(who, n, p, rec, n_acc, cap, ckpt, ckpt_every, ts, ts_ld, K);
   if (rc) return rc;
-  if (lanes < 1 || lanes > 32 || (lanes & (lanes - 1)))
-    return fail(GS_ERR_ARG, std::string(who) + ": lanes must be a power of two up to 32");
+  if (lanes < 0 || lanes > 32 || (lanes & (lanes - 1)) || (lanes == 0 && K > 0))
+    return fail(GS_ERR_ARG, std::string(who) + ": lanes must be a power of two up to 32, or 0 "
+                                               "(two warps) without requested times");
   int D, P;
   if ((rc = field_dims(field, &D, &P))) return rc;
   if (n == 0) return GS_OK;

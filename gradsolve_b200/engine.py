@@ -158,6 +158,7 @@ def first_capacity(n: int, dim: int, max_steps: int, ckpt_every: int, precision:
 # process on a sample of the caller's own trajectories and cached.
 _TUNED: dict = {}
 TUNE_CANDIDATES = (2, 3, 4, 6, 8, 12, 16)
+SAVEAT_CKPT_MAX = 8
 TUNE_MIXED, TUNE_MARGIN_MIXED = 4, 0.04  # (Lotka-Volterra 2^18: K = 2, 3, 4 within 3%, 8 4% off)
 _IN_TUNER = [0]  # nonzero while an autotuner runs its own forwards (no nested tuning)
 
@@ -882,8 +883,13 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw) -> Record:
     if kw["checkpoint"] == "auto" and ok and ws.cap == cap and ws.rec.numel() > 2:
         K = ws.ckpt_every  # sticky: the workspace's interval, so its buffers are reused
     else:
-        K = choose_ckpt_every(kw["checkpoint"], spec.dim, n, cap, kw["budget_bytes"],
-                              tuned_ckpt_every(method, spec, precision))
+        tuned = tuned_ckpt_every(method, spec, precision)
+        if tuned is None and precision == "float64":
+            tuned = 2  # (a batch too small to tune on: its checkpoints are no matter)
+        if saveat_ts is not None and precision == "float64":
+            # (dense output walks K / 2 steps from a checkpoint per requested time)
+            tuned = min(tuned or SAVEAT_CKPT_MAX, SAVEAT_CKPT_MAX)
+        K = choose_ckpt_every(kw["checkpoint"], spec.dim, n, cap, kw["budget_bytes"], tuned)
     yf = ws.y_final if ok else torch.empty_like(y0)
     n_acc, n_rej, status = ((ws.n_acc, ws.n_rej, ws.status) if ok else
                             tuple(torch.empty(n, dtype=torch.int32, device=device)
@@ -1100,35 +1106,45 @@ def _replay_one(r: Record, y0: torch.Tensor, p: torch.Tensor, *, write_ckpt: boo
 
 _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 
-# Lanes per trajectory of the split reverse pass (gs_adjoint_split, csrc/gs_split.cuh), float64
-# states of up to 3 components; 0: one thread per trajectory.  The split costs D (+ 1) step VJPs
-# where one thread takes one, and shortens the chain by the number of lanes: it pays where the
-# batch leaves most of the chip idle, or waits for its longest trajectories.  B200, reverse pass
-# one thread per trajectory / split:
-#   even batches: Lorenz (t = 1, 112 steps) n = 1024 67.6 / 25 us, 4096 67.6 / 39, 16,384 67.8 /
-#   98 (off); Robertson 1024 442 / 45 us;
+# Reverse passes for batches that one thread per trajectory leaves most of the chip idle on, or that
+# wait for their longest trajectories (gs_adjoint_split, float64): the steps of a trajectory
+# split over lanes (csrc/gs_split.cuh, up to 3 components: D (+ 1) step VJPs where one thread
+# takes one, for a chain shorter by the number of lanes), or two warps per 32 trajectories
+# (csrc/gs_paired.cuh, up to 8 components: the one-thread arithmetic).  B200, reverse pass one
+# thread per trajectory / split / two warps:
+#   even batches: Lorenz (t = 1, 112 steps) n = 1024 68 / 25 us, 4096 68 / 39, 8192 48 / - / 29,
+#   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 442 / 45 us, 8192 449 / 197 / 326,
+#   16,384 452 / - / 385; HIRES 8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
 #   per-trajectory end times, 64 saved times: stiff Van der Pol 20,011 9.7 / 1.0 ms (16 lanes),
 #   350,000 18.8 / 7.1; Van der Pol 100,003 1.57 / 0.57 ms (4), 700,000 6.06 / 3.27 (1).
 # The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Even
-# Tsit5 batches take it within SPLIT_EVEN_CAP steps of record: over thousands of steps of an
+# Tsit5 batches are split within SPLIT_EVEN_CAP steps of record: over thousands of steps of an
 # expanding flow (Lorenz, t = 70, gradients of 1e20) the two evaluation orders differ by 1e-8.
 SPLIT_MAX_DIM = 3
-SPLIT_EVEN_MAX = 4096
+SPLIT_EVEN_MAX = {METHOD_TSIT5: 2048, METHOD_ROS23: 8192}
 SPLIT_EVEN_CAP = 4096
 SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without asking for the budget
+PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
 
 
-def split_lanes(n: int, dim: int, even: bool, saveat: bool) -> int:
-    if dim > SPLIT_MAX_DIM or (even and not saveat and n > SPLIT_EVEN_MAX) or (
+def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5) -> int:
+    """Lanes per trajectory of the split reverse pass, 0: not split."""
+    if dim > SPLIT_MAX_DIM or (even and not saveat and n > SPLIT_EVEN_MAX[method]) or (
             not even and not saveat and n > 1 << 17):
         return 0
     room = (1 << 16 if even and not saveat else 1 << 19) // max(n, 1)
     return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
 
 
+def _paired(r) -> bool:
+    """Two warps per 32 trajectories: even batches whose blocks are all resident, short segments."""
+    most = 1 << 14 if r.spec.dim <= 4 else 1 << 13 if r.spec.dim <= 8 else 0
+    return 0 < r.n <= most and not r.uneven and all(rr.ckpt_every <= 2 for _rows, rr in _parts(r))
+
+
 def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> bool:
     if (precision != "float64" or schedule != "auto" or variant != "auto" or
-            not r.y_final.is_cuda or r.spec.dim > SPLIT_MAX_DIM):
+            not r.y_final.is_cuda):
         return False
     key = (r.method, r.spec.key)  # (a pinned occupancy instance is one thread per trajectory)
     return key not in _OCC_REV or _OCC_REV[key] == _OCC_TUNED.get(key)
@@ -1174,13 +1190,15 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
     recomputing kernel's resident threads, else "recompute".  On the float32 route (Tsit5)
     "pairs" runs two trajectories per thread in packed float32x2 arithmetic (built-in
     nonstiff fields), "recompute" one per thread, and "auto" is "pairs" where it is built."""
-    lanes = 0
-    if _split_applies(r, precision, schedule, variant) and (
-            r.uneven or r.method == METHOD_ROS23 or r.cap <= SPLIT_EVEN_CAP):
-        lanes = split_lanes(r.n, r.spec.dim, not r.uneven, False)
+    lanes = None
+    if _split_applies(r, precision, schedule, variant):
+        if r.uneven or r.method == METHOD_ROS23 or r.cap <= SPLIT_EVEN_CAP:
+            lanes = split_lanes(r.n, r.spec.dim, not r.uneven, False, r.method) or None
+        if lanes is None and _paired(r):
+            lanes = PAIRED
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
-    if lanes:
+    if lanes is not None:
         res = _over_parts(r, lambda rr, rows: _adjoint_split(
             rr, lanes, _take(p, rows), _take(ybar, rows).contiguous(), None, None, want_y0,
             want_p, _lane_order(rr, rows is None)))
@@ -1368,7 +1386,7 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
     ``schedule="auto"``, float64, up to 3 components: the split reverse pass; else it refills
     lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
     per trajectory for an even one."""
-    if r.n and _split_applies(r, precision, schedule):
+    if r.n and r.spec.dim <= SPLIT_MAX_DIM and _split_applies(r, precision, schedule):
         words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
         if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
             lanes = split_lanes(r.n, r.spec.dim, not r.uneven, True)

@@ -345,7 +345,9 @@ int gs_adjoint_saveat(int method, int field, int precision, long long n, const d
  * `lanes` times shorter.  Float64, states of up to 3 components (GS_ERR_FIELD above).  work: n *
  * K * (D + P) doubles of scratch.  order: as gs_adjoint_ordered, or NULL.  Gradients agree with
  * the unsplit passes to rounding and depend on neither ckpt_every nor the rest of the batch.
- * No counterpart in the reference.
+ * lanes = 0 (K = 0, states of up to 8 components, segments that fit shared memory): two warps per
+ * 32 trajectories instead, one recomputing the steps' forward quantities a segment ahead of the
+ * other's VJPs -- the unsplit pass's arithmetic.  No counterpart in the reference.
  */
 int gs_adjoint_split(int method, int field, int precision, long long n, const double* p,
                      const double* rec, const int* n_acc, int cap, const double* ckpt,

@@ -66,7 +66,7 @@ def test_split_matches_one_thread(gslib, cuda, method, field):
                     assert torch.equal(a, b), (n, K, lanes)
                 first[lanes] = got
             auto = engine.adjoint(r, p, ybar)
-            lanes = engine.split_lanes(n, spec.dim, False, False)
+            lanes = engine.split_lanes(n, spec.dim, False, False, method)
             if engine._split_applies(r, "float64", "auto"):
                 assert all(torch.equal(a, b) for a, b in zip(auto, first[lanes]))
 
@@ -102,6 +102,48 @@ def test_split_dense_output(gslib, cuda, method, field):
                         assert rowrel(a, b) <= 1e-10, (shared, K, lanes)
 
 
+PAIRED = CASES + [("tsit5", "lorenz96_8"), ("rosenbrock23", "hires")]
+
+
+@pytest.mark.parametrize("method,field", PAIRED)
+def test_two_warps_match_one_thread(gslib, cuda, method, field):
+    """Two warps per 32 trajectories: the one-thread pass's arithmetic, with batches below, at and
+    past a block, trajectories without steps and idle lanes (an order with entries outside)."""
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec = field_spec(field)
+    for n in (1, 32, 33, 70):
+        if field == "hires":
+            y0 = torch.tensor([1.0, 0, 0, 0, 0, 0, 0, 0.0057], device=cuda,
+                              dtype=torch.float64).repeat(n, 1)
+            p = torch.zeros(n, 1, device=cuda, dtype=torch.float64)
+            t1v = torch.linspace(0.0, 5.0, n, device=cuda, dtype=torch.float64)
+        elif field == "lorenz96_8":
+            g = torch.Generator(device=cuda)
+            g.manual_seed(n)
+            p = torch.full((n, 1), 8.0, device=cuda, dtype=torch.float64)
+            y0 = p + torch.rand(n, 8, generator=g, device=cuda, dtype=torch.float64)
+            t1v = torch.linspace(0.0, 1.0, n, device=cuda, dtype=torch.float64)
+        else:
+            y0, p, t1v = _batch(cuda, field, n)
+        for K in (1, 2):
+            r = engine.forward_record(method, spec, y0, p, t0=0.0, t1=10.0, t1v=t1v, rtol=1e-6,
+                                      atol=1e-9, checkpoint=K, max_steps=50000, cap0=50000)
+            ybar = torch.cos(torch.arange(r.y_final.numel(), device=cuda,
+                                          dtype=torch.float64)).reshape(r.y_final.shape)
+            ref = engine.adjoint(r, p, ybar, schedule="static")
+            got = engine._adjoint_split(r, 0, p, ybar, None, None, True, True, None)
+            for a, b in zip(got, ref):
+                assert rowrel(a, b) <= 1e-10, (n, K)
+            order = torch.arange(n - 1, -1, -1, device=cuda)
+            if n > 1:
+                order[0] = n + 5  # an idle lane: trajectory n - 1 is not written
+            part = engine._adjoint_split(r, 0, p, ybar, None, None, True, True, order)
+            for a, b in zip(part, got):
+                m = n - 1 if n > 1 else n
+                assert torch.equal(a[:m], b[:m]), (n, K)
+
+
 def test_split_refuses(gslib, cuda):
     from gradsolve_b200 import engine
     from gradsolve_b200._lib import GsolveError
@@ -111,6 +153,10 @@ def test_split_refuses(gslib, cuda):
                               atol=1e-9, checkpoint=2)
     with pytest.raises(GsolveError, match="power of two"):
         engine._adjoint_split(r, 3, p, r.y_final, None, None, True, True, None)
+    with pytest.raises(GsolveError, match="do not fit"):
+        r64 = engine.forward_record("tsit5", field_spec("lorenz"), y0, p, t0=0.0, t1=1.0,
+                                    rtol=1e-6, atol=1e-9, checkpoint=64)
+        engine._adjoint_split(r64, 0, p, r64.y_final, None, None, True, True, None)
     with pytest.raises(GsolveError, match="cotangent"):
         engine._adjoint_split(r, 2, p, None, None, None, True, True, None)
     spec = field_spec("hires")
