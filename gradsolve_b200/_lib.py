@@ -70,6 +70,11 @@ _SIGS = {
     "gs_adjoint_saveat": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p,
                                   c_int, c_void_p, c_int, c_void_p, c_ll, c_int, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_void_p]),
+    "gs_fwd_compact_bytes": (c_size_t, [c_int, c_int, c_int, c_ll]),
+    "gs_fwd_record_compact": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_double,
+                                      c_void_p, c_double, c_double, c_double, c_double, c_int,
+                                      c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                                      c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "gs_lane_order": (c_int, [c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "gs_adjoint_split": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_int,
                                  c_void_p, c_int, c_int, c_void_p, c_ll, c_int, c_void_p,

@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "../../include/gsolve.h"
+#include "gs_compact.cuh"
 #include "gs_coop.cuh"
 #include "gs_f32.cuh"
 #include "gs_fields.cuh"
@@ -761,6 +762,89 @@ int launch_ros23_adjoint(const gs::AdjointArgs& a, int cap, cudaStream_t s, int 
     return cuda_check("ros23_adjoint_kernel");
   }
   return launch_adjoint_persistent<F, gs::Ros23Step>(a, cap, s, sched == GS_SCHED_REFILL);
+}
+
+// ---- recording forward with compaction (gs_compact.cuh) ----------------------------------
+constexpr size_t kCompactHead = 256;  // the lists' counters
+
+template <class F>
+constexpr bool kCompactBuilt = F::D <= 4;
+
+// Two lists that the passes fill in turn: what pass 0 and pass 1 can leave behind.
+template <class M>
+size_t compact_bytes(long long n) {
+  return kCompactHead + (size_t)(gs::compact_left(n, 0) + gs::compact_left(n, 1)) *
+                            gs::compact_words<M>() * sizeof(double);
+}
+
+template <class F, class M, int kMinB>
+int launch_compact(const gs::RecordArgs& a_in, void* work, size_t bytes, cudaStream_t s) {
+  if (!work || bytes < compact_bytes<M>(a_in.n))
+    return fail(GS_ERR_ARG, "gs_fwd_record_compact: work is smaller than gs_fwd_compact_bytes");
+  gs::RecordArgs a = a_in;
+  a.ctrl = gs::make_ctrl_consts(F::D, M::QK);
+  cudaError_t e = cudaMemsetAsync(work, 0, kCompactHead, s);
+  if (e != cudaSuccess)
+    return fail(GS_ERR_CUDA, std::string("CUDA: cudaMemsetAsync: ") + cudaGetErrorString(e));
+  int* counts = static_cast<int*>(work);
+  double* list[2];
+  list[0] = reinterpret_cast<double*>(static_cast<unsigned char*>(work) + kCompactHead);
+  list[1] = list[0] + gs::compact_left(a.n, 0) * gs::compact_words<M>();
+  gs::CompactLists l{nullptr, nullptr, nullptr, nullptr, 0, 0};
+  long long threads = a.n;
+  for (int pass = 0; pass < gs::kPasses; ++pass) {
+    const bool last = pass + 1 == gs::kPasses;
+    l.out = last ? nullptr : list[pass & 1];
+    l.out_count = counts + pass;
+    l.out_cap = gs::compact_left(a.n, pass);
+    gs::record_compact_kernel<F, M, kMinB><<<grid_for(threads), kBlock, 0, s>>>(a, l);
+    int rc = cuda_check("record_compact_kernel");
+    if (rc) return rc;
+    l.in = l.out;
+    l.in_count = l.out_count;
+    l.in_cap = l.out_cap;
+    threads = l.in_cap;
+  }
+  return GS_OK;
+}
+
+template <class F>
+int compact_size(int prec, int method, long long n, size_t* bytes) {
+  if constexpr (!kCompactBuilt<F>) {
+    (void)prec; (void)method; (void)n;
+    *bytes = 0;
+  } else {
+    *bytes = method == GS_METHOD_ROS23  ? compact_bytes<gs::CompactRos23<F>>(n)
+             : prec == GS_PREC_MIXED    ? compact_bytes<gs::CompactMixed<F>>(n)
+                                        : compact_bytes<gs::CompactTsit5<F>>(n);
+  }
+  return GS_OK;
+}
+
+template <class F>
+int compact_refuse() {
+  return fail(GS_ERR_FIELD, "gs_fwd_record_compact: built for states of up to 4 components, not "
+                            "D = " + std::to_string(F::D));
+}
+template <class F>
+int launch_compact_tsit5(const gs::RecordArgs& a, int prec, void* work, size_t bytes,
+                         cudaStream_t s) {
+  if constexpr (!kCompactBuilt<F>) {
+    (void)a; (void)prec; (void)work; (void)bytes; (void)s;
+    return compact_refuse<F>();
+  } else {
+    return prec == GS_PREC_MIXED ? launch_compact<F, gs::CompactMixed<F>, 1>(a, work, bytes, s)
+                                 : launch_compact<F, gs::CompactTsit5<F>, 6>(a, work, bytes, s);
+  }
+}
+template <class F>
+int launch_compact_ros23(const gs::RecordArgs& a, void* work, size_t bytes, cudaStream_t s) {
+  if constexpr (!kCompactBuilt<F>) {
+    (void)a; (void)work; (void)bytes; (void)s;
+    return compact_refuse<F>();
+  } else {
+    return launch_compact<F, gs::CompactRos23<F>, 1>(a, work, bytes, s);
+  }
 }
 
 // ---- the float32 route (GS_PREC_F32, gs_f32.cuh) ----------------------------------------
@@ -1907,6 +1991,46 @@ extern "C" int gs_adjoint_split(int method, int field, int precision, long long 
   }
   if (method == GS_METHOD_ROS23) {
     GS_ROS23_DISPATCH(field, launch_split_ros23, a, s, lanes, work, order)
+  }
+  return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
+}
+
+extern "C" size_t gs_fwd_compact_bytes(int method, int field, int precision, long long n) {
+  size_t bytes = 0;
+  auto size = [&]() -> int {
+    GS_TSIT5_DISPATCH(field, compact_size, precision & GS_PREC_MASK, method, n, &bytes)
+  };
+  return n > 0 && n <= 0x7fffffffll && size() == GS_OK ? bytes : 0;
+}
+
+extern "C" int gs_fwd_record_compact(int method, int field, int precision, long long n,
+                                     const double* y0, const double* p, double t0,
+                                     const double* t1v, double t1, double rtol, double atol,
+                                     double dt0, int max_steps, int cap, int ckpt_every,
+                                     double* rec, double* ckpt, double* y_final, int* n_acc,
+                                     int* n_rej, int* status, void* work, size_t work_bytes,
+                                     void* stream) {
+  const char* who = "gs_fwd_record_compact";
+  if (precision != GS_PREC_F64 && !(precision == GS_PREC_MIXED && method == GS_METHOD_TSIT5))
+    return fail(GS_ERR_PRECISION, std::string(who) + ": float64, or float32 stages with Tsit5, "
+                                                     "without flags");
+  int rc = check_record_args(who, n, y0, p, rtol, atol, max_steps, cap, ckpt_every, rec, ckpt,
+                             y_final, n_acc, n_rej, status);
+  if (rc) return rc;
+  int D, P;
+  if ((rc = field_dims(field, &D, &P))) return rc;
+  if (n == 0) return GS_OK;
+  if (!rec || !ckpt || n > 0x7fffffffll || !aligned16(work))
+    return fail(GS_ERR_ARG, std::string(who) + ": rec, ckpt and an aligned work are required, for "
+                                               "up to 2^31 - 1 trajectories");
+  gs::RecordArgs a{n, y0, p, t0, t1, rtol, atol, dt0, t1v, max_steps, cap, ckpt_every,
+                   gs_ckpt_slots(cap, ckpt_every), rec, ckpt, y_final, n_acc, n_rej, status};
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (method == GS_METHOD_TSIT5) {
+    GS_TSIT5_DISPATCH(field, launch_compact_tsit5, a, precision, work, work_bytes, s)
+  }
+  if (method == GS_METHOD_ROS23) {
+    GS_ROS23_DISPATCH(field, launch_compact_ros23, a, work, work_bytes, s)
   }
   return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
 }

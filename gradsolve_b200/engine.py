@@ -606,6 +606,7 @@ def _lanes_flag(method: str, spec: FieldSpec) -> int:
 # the field and is measured once per process on a sample of the caller's trajectories.
 _OCC: dict = {}      # (method, field key) -> GS_OCC blocks per SM of the forward (0: default)
 _OCC_REV: dict = {}  # (method, field key) -> the same for the reverse pass at K = 2
+_OCC_PINNED: set = set()  # (method, field key) whose forward's instance set_occupancy pinned
 _OCC_TUNED: dict = {}  # the autotuner's own entries of _OCC_REV (an entry that differs is a pin)
 OCC_MARGIN = 0.01    # another instance replaces the default only when faster by more than 1%
 MIXED = "tsit5/mixed"  # the tables' method key of the Tsit5 float32-stage reverse pass
@@ -632,6 +633,8 @@ def set_occupancy(spec: FieldSpec, blocks: Optional[int], pass_: str = "forward"
     table = _OCC if pass_ == "forward" else _OCC_REV
     if pass_ == "reverse":
         _OCC_TUNED.pop((method, spec.key), None)  # what the table holds from here on is a pin
+    else:
+        (_OCC_PINNED.discard if blocks is None else _OCC_PINNED.add)((method, spec.key))
     if blocks is None:
         table.pop((method, spec.key), None)
         return
@@ -868,13 +871,39 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
                          ws.n_rej, ws.status, uneven=ws.uneven, ys=ws.ys, streams=[None])
         return _forward_planned(method, spec, y0, p, t1v, saveat_ts, plan, kw)
     cap = max(1, min(int(cap0), int(max_steps)))
-    r0 = _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw)
+    r0 = _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw,
+                      compact=_compacts(method, spec, n, precision, schedule, t1v, saveat_ts))
     return _grow(method, spec, y0, p, t1v, saveat_ts, r0, None, kw)
 
 
-def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw) -> Record:
+# Fresh batches from these sizes up run the compacting forward (gs_fwd_record_compact,
+# csrc/gs_compact.cuh): their step counts are not known yet, and where they spread a third of the
+# one-launch forward's lanes idle.  Below, its launches' tails cost what it saves: Robertson 65,536
+# 1.06 / 1.00 ms, Lotka-Volterra (float32 stages) 65,536 137 / 164 us, 2^18 388 / 374 us.
+COMPACT_MIN = {METHOD_TSIT5: 1 << 18, METHOD_ROS23: 1 << 16}
+COMPACT_MAX_DIM = 4
+
+
+def _compacts(method, spec, n, precision, schedule, t1v, saveat_ts) -> bool:
+    return (n >= COMPACT_MIN[method] and spec.dim <= COMPACT_MAX_DIM and schedule == "auto" and
+            t1v is None and saveat_ts is None and (method, spec.key) not in _OCC_PINNED and
+            not _IN_TUNER[0] and
+            (precision == "float64" or (precision == "mixed" and method == METHOD_TSIT5)))
+
+
+def _compact_work(L, code, n, device) -> Optional[torch.Tensor]:
+    """Scratch of the compacting forward, 30 to 80 bytes a trajectory; None where it does not
+    fit (the one-launch forward needs none)."""
+    size = L.gs_fwd_compact_bytes(*code, n)
+    try:
+        return torch.empty(size, dtype=torch.uint8, device=device) if size else None
+    except torch.OutOfMemoryError:
+        return None
+
+
+def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False) -> Record:
     """One record of capacity ``cap`` for all rows of y0 (buffers reused from ws if they
-    match), on the current stream."""
+    match), on the current stream; ``compact``: by the compacting forward."""
     n = y0.shape[0]
     device = y0.device
     L = _lib.lib_for(spec)
@@ -906,8 +935,12 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw) -> Record:
             dt0_arg, int(kw["max_steps"]), cap, K, _ptr(rec), _ptr(ckpt), _ptr(yf),
             _ptr(n_acc), _ptr(n_rej), _ptr(status))
     ys = None
+    code = (_METHOD_CODE[method], spec.code, _PREC[precision])
     if n == 0:
         pass
+    elif compact and (work := _compact_work(L, code, n, device)) is not None:
+        _lib.check(L.gs_fwd_record_compact(*code, n, _ptr(y0), _ptr(p), *args, _ptr(work),
+                                           work.numel(), _stream()), "gs_fwd_record_compact", L)
     elif saveat_ts is None:
         fn = L.gs_tsit5_fwd_record if method == METHOD_TSIT5 else L.gs_ros23_fwd_record
         _lib.check(fn(spec.code, mode, n, _ptr(y0), _ptr(p), *args, _stream()), fn.__name__, L)

@@ -222,6 +222,21 @@ int gs_tsit5_fwd_record(int field, int precision, long long n, const double* y0,
                         int* status, void* stream);
 
 /*
+ * The recording forward of gs_tsit5_fwd_record (float64 or float32 stages) / gs_ros23_fwd_record
+ * for a large batch whose step counts are not known and spread: warps with few unfinished
+ * trajectories left hand them to a further launch that takes them with full warps
+ * (csrc/gs_compact.cuh).  States of up to 4 components; rec and ckpt are required; work:
+ * gs_fwd_compact_bytes bytes of scratch, 16-byte aligned.  Results are those of the one-launch
+ * forward, trajectory by trajectory.  No counterpart in the reference.
+ */
+size_t gs_fwd_compact_bytes(int method, int field, int precision, long long n);
+int gs_fwd_record_compact(int method, int field, int precision, long long n, const double* y0,
+                          const double* p, double t0, const double* t1v, double t1, double rtol,
+                          double atol, double dt0, int max_steps, int cap, int ckpt_every,
+                          double* rec, double* ckpt, double* y_final, int* n_acc, int* n_rej,
+                          int* status, void* work, size_t work_bytes, void* stream);
+
+/*
  * Frozen-mesh replay: re-integrate n_acc[j] recorded steps of trajectory j with fixed
  * steps.  Replaces gradsolve/warp/warp_replay.py:30-55 (replay_solve_jax) over
  * gradsolve/solvers/tsit5_step.py:80-102 (tsit5_step).  Optionally writes checkpoints
