@@ -21,7 +21,8 @@
 // other trajectories share the batch; against one thread per trajectory they agree to rounding.
 //
 // B200, stiff Van der Pol batch (20,011 trajectories, 2269 steps on average, 17,220 the longest,
-// 64 saved times): forward with inline re-steps 14.0 ms, reverse pass 9.9 ms one lane each.
+// 64 saved times): reverse pass 9.9 ms with one lane each, 1.0 ms with 16; the whole closure
+// (with a record that holds every step at once) 48.9 -> 11.2 ms.
 #pragma once
 #include <math_constants.h>
 

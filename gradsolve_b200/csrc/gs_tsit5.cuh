@@ -713,7 +713,8 @@ __device__ __forceinline__ bool tsit5_attempt(const RecordArgs& a, long long j,
 // Bounded to 6 resident blocks of 128 per SM (80 registers) for D <= 4: with the
 // shared-reciprocal error norm the unbounded kernel takes 84 and drops to 5 blocks; the few
 // bytes it spills at 80 cost less than the lost warps (11.63 vs 11.73 ms on the Lorenz 2^20
-// bench forward; 7 blocks at 72 registers: 11.35 ms).  Larger states keep their registers.
+// bench forward when this bound was set; the occupancy autotuner measures the others per field,
+// and the same forward now takes 9.9 ms).  Larger states keep their registers.
 // kStore = false: the forward-only solve (no record, no checkpoints), with the store paths
 // compiled out.  kMinB > 0 bounds the registers for kMinB resident blocks per SM instead
 // (the instances the occupancy autotuner chooses among; same arithmetic, bit for bit).

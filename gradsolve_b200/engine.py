@@ -1190,7 +1190,6 @@ def _adjoint_split(r: Record, lanes: int, p, ybar, ts, ysbar, want_y0, want_p, o
     gy0 = torch.empty((r.n, D), dtype=torch.float64, device=dev) if want_y0 else None
     gp = torch.empty((r.n, p.shape[1]), dtype=torch.float64, device=dev) if want_p else None
     ld = K = 0
-    work = None
     if ts is not None:
         ts, ld, K = _ts_arg(ts, r.n)
         if work is None:

@@ -72,7 +72,7 @@ extern "C" {
  * the next trajectory from a work counter when theirs finishes (uneven batches; the counter
  * lives in the checkpoint buffer's control block).  STRIDED: persistent lanes taking
  * trajectories j, j+G, ...  AUTO (0): STATIC, except REFILL for a forward with per-trajectory
- * end times. */
+ * end times and more trajectories than the chip holds threads at once. */
 #define GS_SCHED_AUTO 0x000
 #define GS_SCHED_STATIC 0x100
 #define GS_SCHED_REFILL 0x200
@@ -326,8 +326,8 @@ int gs_replay_saveat(int method, int field, int precision, long long n, const do
  * rounding (the same step function, compiled into another kernel).  Schedules: lanes refilled
  * from a work counter (GS_SCHED_REFILL, or AUTO when trajectories have their own end times and
  * are more than the chip holds at once; needs ckpt), persistent strided lanes
- * (GS_SCHED_STRIDED), one thread per trajectory otherwise (GS_SCHED_STATIC, or AUTO).  No counterpart in the reference,
- * whose saveat always replays the recorded mesh (gradsolve/warp/warp_replay.py:58-84).
+ * (GS_SCHED_STRIDED), one thread per trajectory otherwise (GS_SCHED_STATIC, or AUTO).  No
+ * counterpart in the reference, whose saveat always replays the recorded mesh (gradsolve/warp/warp_replay.py:58-84).
  * method: GS_METHOD_TSIT5 (float64 or mixed) or GS_METHOD_ROS23 (float64).
  */
 int gs_fwd_record_saveat(int method, int field, int precision, long long n, const double* y0,

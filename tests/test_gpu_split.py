@@ -166,3 +166,24 @@ def test_split_refuses(gslib, cuda):
                                checkpoint=2)
     with pytest.raises(GsolveError, match="up to 3 components"):
         engine._adjoint_split(r8, 2, p8, r8.y_final, None, None, True, True, None)
+
+
+def test_split_dense_output_takes_one_workspace(gslib, cuda):
+    """adjoint_saveat's scratch is one word per requested time and gradient component, once."""
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    n, K, spec = 4096, 64, field_spec("vdp")
+    rng = np.random.default_rng(5)
+    y0 = torch.tensor(rng.uniform(-2, 2, (n, 2)), device=cuda)
+    p = torch.tensor(rng.uniform(0.1, 5.0, (n, 1)), device=cuda)
+    ts = torch.linspace(0.0, 2.0, K, device=cuda, dtype=torch.float64)
+    r = engine.forward_record("tsit5", spec, y0, p, t0=0.0, t1=2.0, rtol=1e-6, atol=1e-9,
+                              saveat_ts=ts)
+    bar = torch.ones_like(r.ys)
+    engine.adjoint_saveat(r, p, ts, bar)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    engine.adjoint_saveat(r, p, ts, bar)
+    work = 8 * n * K * (2 + 1)
+    assert torch.cuda.max_memory_allocated() - before < 1.5 * work
