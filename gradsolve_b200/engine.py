@@ -1149,12 +1149,17 @@ _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 #   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 442 / 45 us, 8192 449 / 197 / 326,
 #   16,384 452 / - / 385; HIRES 8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
 #   per-trajectory end times, 64 saved times: stiff Van der Pol 20,011 9.7 / 1.0 ms (16 lanes),
-#   350,000 18.8 / 7.1; Van der Pol 100,003 1.57 / 0.57 ms (4), 700,000 6.06 / 3.27 (1).
+#   200,000 11.8 / 9.9, 350,000 11.8 / 20.1; Van der Pol 100,000 1.37 / 0.67 ms (4), 200,000
+#   1.73 / 1.15, 350,000 1.66 / 2.01, 700,000 2.60 / 3.57 (one thread: lanes refilled);
+#   even batches, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
+#   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 392 / 230, 16,384
+#   409 / 667, 262,144 2.08 / 4.94 ms.
 # The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Even
 # Tsit5 batches are split within SPLIT_EVEN_CAP steps of record: over thousands of steps of an
 # expanding flow (Lorenz, t = 70, gradients of 1e20) the two evaluation orders differ by 1e-8.
 SPLIT_MAX_DIM = 3
 SPLIT_EVEN_MAX = {METHOD_TSIT5: 2048, METHOD_ROS23: 8192}
+SPLIT_EVEN_SAVEAT_MAX = 4096
 SPLIT_EVEN_CAP = 4096
 SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without asking for the budget
 PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
@@ -1162,8 +1167,11 @@ PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
 
 def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5) -> int:
     """Lanes per trajectory of the split reverse pass, 0: not split."""
-    if dim > SPLIT_MAX_DIM or (even and not saveat and n > SPLIT_EVEN_MAX[method]) or (
-            not even and not saveat and n > 1 << 17):
+    if even:
+        most = SPLIT_EVEN_SAVEAT_MAX if saveat else SPLIT_EVEN_MAX[method]
+    else:
+        most = 1 << (18 if saveat else 17)
+    if dim > SPLIT_MAX_DIM or n > most:
         return 0
     room = (1 << 16 if even and not saveat else 1 << 19) // max(n, 1)
     return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
@@ -1415,13 +1423,13 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
                    ybar: Optional[torch.Tensor] = None, *, want_y0: bool = True,
                    want_p: bool = True, precision: str = "float64", schedule: str = "auto"):
     """(dL/dy0, dL/dp) for cotangents ysbar = dL/dys (n, K, D) and ybar = dL/dy_final.
-    ``schedule="auto"``, float64, up to 3 components: the split reverse pass; else it refills
+    ``schedule="auto"``, float64, where split_lanes says so: the split reverse pass; else it refills
     lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
     per trajectory for an even one."""
-    if r.n and r.spec.dim <= SPLIT_MAX_DIM and _split_applies(r, precision, schedule):
+    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, True)
+    if r.n and lanes and _split_applies(r, precision, schedule):
         words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
         if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
-            lanes = split_lanes(r.n, r.spec.dim, not r.uneven, True)
             f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
             # the workspaces come from the caller's stream's pool (a side stream's would be empty
             # on its first use): _over_parts orders the side streams after it and it after them,
