@@ -203,6 +203,14 @@ __global__ void __launch_bounds__(128) saveat_vjp_kernel(const SaveatArgs a, dou
   }
 }
 
+// The recorded steps a pass takes: those of the replay whose checkpoints it reads.  Dense output
+// walks forward in time (gs_saveat.cuh); the plain replay takes every step that is not 0, so a
+// mesh given by the caller may also step backwards, and a NaN step makes the gradient NaN.
+template <bool kSave>
+__device__ __forceinline__ bool takes_step(double dt) {
+  return kSave ? dt > 0.0 : dt != 0.0;
+}
+
 // ---- the split reverse pass ------------------------------------------------------------------
 // G lanes (a power of two, at most 32) per trajectory; order: as AdjointArgs.  kSave: with the
 // cotangents of dense output (a.ts, a.ysbar, work of saveat_vjp_kernel).
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
       for (int i = 0; i < D; ++i) buf.st(q, i) = y[i];
       buf.st(q, D) = t;
       const double dt = buf.dt(b, q);
-      if (dt > 0.0) {
+      if (takes_step<kSave>(dt)) {
         if (q + 1 < q1) {
           double cy[D];
 #pragma unroll
@@ -284,7 +292,7 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
     }
     for (int q = q1 - 1; q >= q0; --q) {
       const double dt = buf.dt(b, q);
-      if (dt > 0.0) {
+      if (takes_step<kSave>(dt)) {
         double ys[D];
 #pragma unroll
         for (int i = 0; i < D; ++i) ys[i] = buf.st(q, i);

@@ -187,3 +187,34 @@ def test_split_dense_output_takes_one_workspace(gslib, cuda):
     engine.adjoint_saveat(r, p, ts, bar)
     work = 8 * n * K * (2 + 1)
     assert torch.cuda.max_memory_allocated() - before < 1.5 * work
+
+
+@pytest.mark.parametrize("method,field", [("tsit5", "lorenz"), ("tsit5", "vdp"),
+                                          ("rosenbrock23", "vdp")])
+def test_split_takes_the_replays_steps(gslib, cuda, method, field):
+    """A caller's mesh may step backwards or hold a NaN step: the replay takes those steps, and so
+    does the reverse pass on both sides of the size from which one thread takes a trajectory."""
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec = field_spec(field)
+    most = engine.SPLIT_EVEN_MAX[method]
+    for n in (37, most, most + 1):
+        y0, p, _t1v = _batch(cuda, field, n)
+        dts = torch.full((n, 40), 0.02, device=cuda, dtype=torch.float64)
+        dts[:, 7::9] = -1e-4
+        for K in (1, 3):
+            r = engine.record_from_padded(method, spec, dts, 0.0, checkpoint=K)
+            yf = engine.replay(r, y0, p)
+            ybar = 1.0 + torch.cos(torch.arange(yf.numel(), device=cuda,
+                                                dtype=torch.float64)).reshape(yf.shape)
+            ref = engine.adjoint(r, p, ybar, schedule="static")
+            for a, b in zip(engine.adjoint(r, p, ybar), ref):
+                assert rowrel(a, b) <= 1e-10, (n, K)
+        dts[1, 5] = float("nan")
+        r = engine.record_from_padded(method, spec, dts, 0.0, checkpoint=3)
+        yf = engine.replay(r, y0, p)
+        gy0, gp = engine.adjoint(r, p, ybar)
+        assert bool(gy0[1].isnan().all()) and bool(gp[1].isnan().any()), n
+        keep = torch.arange(n, device=cuda) != 1  # the other trajectories are as they were
+        for a, b in zip((gy0, gp), ref):
+            assert rowrel(a[keep], b[keep]) <= 1e-10, n
