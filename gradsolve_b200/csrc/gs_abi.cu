@@ -294,7 +294,7 @@ int zero_counter(unsigned long long* c, cudaStream_t s) {
 template <class F, class L>
 int launch_record_persistent(const gs::RecordArgs& a_in, cudaStream_t s, bool use_counter) {
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, L::QK);
+  a.ctrl = gs::make_ctrl_consts(F::D, L::QK, a.rtol, a.atol);
   unsigned long long* counter =
       use_counter ? ctrl_counter(a.ckpt, a.n, a.ck_slots, F::D, gs::kCtrlFwd) : nullptr;
   unsigned grid = 0;
@@ -468,7 +468,7 @@ template <class F>
 int launch_coop_record(const gs::RecordArgs& a_in, cudaStream_t s, bool mixed, int precision) {
   if (mixed) return coop_refuse_mixed();
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, 10);
+  a.ctrl = gs::make_ctrl_consts(F::D, 10, a.rtol, a.atol);
   return with_lanes<F>(precision, [&](auto g) {
     constexpr int G = decltype(g)::value;
     const unsigned grid = grid_for(a.n * G);
@@ -521,7 +521,7 @@ int launch_tsit5_record(const gs::RecordArgs& a_in, cudaStream_t s, bool mixed, 
   if (precision & GS_LANES_MASK)
     return fail(GS_ERR_ARG, "lanes per trajectory apply to fields of more than 8 components only");
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, 10);  // Tsit5: err^(-1/5) = m^(-1/10)
+  a.ctrl = gs::make_ctrl_consts(F::D, 10, a.rtol, a.atol);  // Tsit5: err^(-1/5) = m^(-1/10)
   const int occ = (precision & GS_OCC_MASK) >> GS_OCC_SHIFT;
   if (occ && (mixed || sched != GS_SCHED_STATIC || (!a.rec && !a.ckpt)))
     return fail(GS_ERR_ARG, "GS_OCC applies to the float64 recording forward, one thread per "
@@ -660,7 +660,7 @@ template <class F>
 int launch_ros23_record(const gs::RecordArgs& a_in, cudaStream_t s, int sched, int precision) {
   const int occ = (precision & GS_OCC_MASK) >> GS_OCC_SHIFT;
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, 6);  // Rosenbrock23: err^(-1/3) = m^(-1/6)
+  a.ctrl = gs::make_ctrl_consts(F::D, 6, a.rtol, a.atol);  // Rosenbrock23: err^(-1/3) = m^(-1/6)
   if (occ && (sched != GS_SCHED_STATIC || (!a.rec && !a.ckpt)))
     return fail(GS_ERR_ARG, "GS_OCC applies to the float64 recording forward, one thread per "
                             "trajectory");
@@ -782,7 +782,7 @@ int launch_compact(const gs::RecordArgs& a_in, void* work, size_t bytes, cudaStr
   if (!work || bytes < compact_bytes<M>(a_in.n))
     return fail(GS_ERR_ARG, "gs_fwd_record_compact: work is smaller than gs_fwd_compact_bytes");
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, M::QK);
+  a.ctrl = gs::make_ctrl_consts(F::D, M::QK, a.rtol, a.atol);
   cudaError_t e = cudaMemsetAsync(work, 0, kCompactHead, s);
   if (e != cudaSuccess)
     return fail(GS_ERR_CUDA, std::string("CUDA: cudaMemsetAsync: ") + cudaGetErrorString(e));
@@ -1754,7 +1754,7 @@ template <class F, class L>
 int launch_fwd_lanes(const gs::RecordArgs& a_in, cudaStream_t s, FwdLanes lanes) {
   if (lanes != kStatic) return launch_record_persistent<F, L>(a_in, s, lanes == kRefill);
   gs::RecordArgs a = a_in;
-  a.ctrl = gs::make_ctrl_consts(F::D, L::QK);
+  a.ctrl = gs::make_ctrl_consts(F::D, L::QK, a.rtol, a.atol);
   gs::record_static_kernel<F, L><<<grid_for(a.n), kBlock, 0, s>>>(a);
   return cuda_check("record_static_kernel");
 }

@@ -127,7 +127,7 @@ __device__ __forceinline__ bool tsit5_coop_attempt(const RecordArgs& a, long lon
   tsit5_k2_to_k6<L>(y, p, k1, h, S);
   tsit5_y5<L>(y, k1, S, h, yo);
   L::rhs(yo, p, ko);
-  double part = 0.0;
+  double part = 0.0, ev[C];
 #pragma unroll
   for (int i = 0; i < C; ++i) {
     const double e = h * (T::E1 * k1[i] + T::E2 * S.k2[i] + T::E3 * S.k3[i] + T::E4 * S.k4[i] +
@@ -135,11 +135,21 @@ __device__ __forceinline__ bool tsit5_coop_attempt(const RecordArgs& a, long lon
     const double sc = a.atol + a.rtol * fmax(fabs(y[i]), fabs(yo[i]));
     const double q = e * reciprocal(sc);
     part += q * q;
+    ev[i] = e;
   }
-  const double m = L::sum(part);
-  if (!(m == m)) {  // NaN error: dt would turn NaN and the loop could never finish
-    c.st = 1;
-    return false;
+  double m = L::sum(part);
+  if (!(m < a.ctrl.sum_limit)) {  // as norm_failed (m is the group's: its lanes go together)
+    part = 0.0;
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const double q = ev[i] / (a.atol + a.rtol * fmax(fabs(y[i]), fabs(yo[i])));
+      part += q * q;
+    }
+    m = L::sum(part);
+    if (!(m == m)) {
+      c.st = 1;
+      return false;
+    }
   }
   if (m <= a.ctrl.accept_sum) {
     if ((rec_on || ck_on) && c.acc >= a.cap) {

@@ -307,8 +307,8 @@ __device__ __forceinline__ bool mixed_attempt(const RecordArgs& a, long long j, 
     ed[i] = (double)(hf * (T::E2 * S.dk2[i] + T::E3 * S.dk3[i] + T::E4 * S.dk4[i] +
                            T::E5 * S.dk5[i] + T::E6 * S.dk6[i] + T::E7 * dk7));
   }
-  const double m = wrms_sumsq<D>(ed, y, yo, a.rtol, a.atol);
-  if (!(m == m)) {
+  double m = wrms_sumsq<D>(ed, y, yo, a.rtol, a.atol);
+  if (norm_failed<D>(m, ed, y, yo, a)) {
     ct.st = 1;
     return false;
   }

@@ -55,9 +55,9 @@ struct LaneTsit5F64 {
   __device__ __forceinline__ void start(const double* y, const double* p, const float*) {
     F::rhs(y, p, k1);
   }
-  // candidate y5 for step h; returns the sum of squares of the scaled error
-  __device__ __forceinline__ double trial(const double* y, const double* p, const float*, double h,
-                                          double rtol, double atol, double* y5) {
+  // candidate y5 for step h and the sum of squares m of the scaled error; false: it is NaN
+  __device__ __forceinline__ bool trial(const RecordArgs& a, const double* y, const double* p,
+                                        const float*, double h, double* y5, double& m) {
     using T = Tsit5;
     Stages<F> S;
     double e[D];
@@ -68,7 +68,8 @@ struct LaneTsit5F64 {
     for (int i = 0; i < D; ++i)
       e[i] = h * (T::E1 * k1[i] + T::E2 * S.k2[i] + T::E3 * S.k3[i] + T::E4 * S.k4[i] +
                   T::E5 * S.k5[i] + T::E6 * S.k6[i] + T::E7 * k7[i]);
-    return wrms_sumsq<D>(e, y, y5, rtol, atol);
+    m = wrms_sumsq<D>(e, y, y5, a.rtol, a.atol);
+    return !norm_failed<D>(m, e, y, y5, a);
   }
   __device__ __forceinline__ void commit() {
 #pragma unroll
@@ -87,8 +88,8 @@ struct LaneTsit5Mixed {
 #pragma unroll
     for (int i = 0; i < D; ++i) c[i] = 0.0;
   }
-  __device__ __forceinline__ double trial(const double* y, const double* p, const float* pf,
-                                          double h, double rtol, double atol, double* y5) {
+  __device__ __forceinline__ bool trial(const RecordArgs& a, const double* y, const double* p,
+                                        const float* pf, double h, double* y5, double& m) {
     using T = Tsit5f;
     const float hf = (float)h;
     float yf[D], k1f[D];
@@ -108,7 +109,8 @@ struct LaneTsit5Mixed {
       ed[i] = (double)(hf * (T::E2 * S.dk2[i] + T::E3 * S.dk3[i] + T::E4 * S.dk4[i] +
                              T::E5 * S.dk5[i] + T::E6 * S.dk6[i] + T::E7 * dk7));
     }
-    return wrms_sumsq<D>(ed, y, y5, rtol, atol);
+    m = wrms_sumsq<D>(ed, y, y5, a.rtol, a.atol);
+    return !norm_failed<D>(m, ed, y, y5, a);
   }
   __device__ __forceinline__ void commit() {
 #pragma unroll
@@ -122,11 +124,12 @@ struct LaneRos23 {
   static constexpr int D = F::D, QK = 6;
   using Step = Ros23Step;
   __device__ __forceinline__ void start(const double*, const double*, const float*) {}
-  __device__ __forceinline__ double trial(const double* y, const double* p, const float*, double h,
-                                          double rtol, double atol, double* ynew) {
+  __device__ __forceinline__ bool trial(const RecordArgs& a, const double* y, const double* p,
+                                        const float*, double h, double* ynew, double& m) {
     double ev[D];
     ros23_trial<F>(y, p, h, ynew, ev);
-    return wrms_sumsq<D, false>(ev, y, ynew, rtol, atol);
+    m = wrms_sumsq<D, false>(ev, y, ynew, a.rtol, a.atol);
+    return !norm_failed<D, false>(m, ev, y, ynew, a);
   }
   __device__ __forceinline__ void commit() {}
   // the step no longer advances time: status 2 (gradsolve/solvers/record_jax.py:109)
@@ -199,8 +202,8 @@ __global__ void __launch_bounds__(128) record_static_kernel(const RecordArgs a) 
       st = 2;
       break;
     }
-    const double m = lane.trial(y, p, pf, h, a.rtol, a.atol, ynew);
-    if (!(m == m)) {
+    double m;
+    if (!lane.trial(a, y, p, pf, h, ynew, m)) {
       st = 1;
       break;
     }
@@ -315,9 +318,10 @@ __global__ void __launch_bounds__(128) record_persistent_kernel(const RecordArgs
       if (lane.degenerate(t, h)) {
         st = 2;
       } else {
-        const double m = lane.trial(y, p, pf, h, a.rtol, a.atol, ynew);
+        double m;
+        const bool ok = lane.trial(a, y, p, pf, h, ynew, m);
         ++it;
-        if (!(m == m)) {
+        if (!ok) {
           st = 1;
         } else if (m <= a.ctrl.accept_sum) {
           if ((rec_on || ck_on) && acc >= a.cap) {

@@ -57,7 +57,7 @@ extern "C" int gs_probe_step_factor(const double* S, long long n, int order, int
                                     void* stream) {
   if (n <= 0) return 0;
   if (D < 1 || (order != 5 && order != 3)) return -1;
-  const gs::CtrlConsts c = gs::make_ctrl_consts(D, order == 5 ? 10 : 6);
+  const gs::CtrlConsts c = gs::make_ctrl_consts(D, order == 5 ? 10 : 6, 1e-6, 1e-9);
   step_factor_probe<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       S, n, order, D, c, fast, ref, accept_fast, accept_ref);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -424,24 +424,6 @@ __device__ __forceinline__ void ros23_core(const R* y, const R* p, R h, RosCore<
   ros23_core_as<F, false>(y, p, h, c, ynew);
 }
 
-// Vectors by value, for the out-of-line steps (no address of a register array is taken).
-template <int N>
-struct DVec {
-  double v[N];
-};
-template <int N>
-__device__ __forceinline__ DVec<N> to_dvec(const double* a) {
-  DVec<N> r;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.v[i] = a[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ void from_dvec(const DVec<N>& r, double* a) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) a[i] = r.v[i];
-}
-
 // One attempt of the adaptive forward: the candidate yo and the error vector ev.
 template <class F, bool kSparse>
 __device__ __forceinline__ bool ros23_trial_as(const double* y, const double* p, double h,
@@ -617,8 +599,8 @@ __device__ __forceinline__ bool ros23_attempt(const RecordArgs& a, long long j, 
   ++c.it;
   double ev[D];
   ros23_trial<F>(y, p, h, yo, ev);
-  const double m = wrms_sumsq<D, false>(ev, y, yo, a.rtol, a.atol);
-  if (!(m == m)) {
+  double m = wrms_sumsq<D, false>(ev, y, yo, a.rtol, a.atol);
+  if (norm_failed<D, false>(m, ev, y, yo, a)) {
     c.st = 1;
     return false;
   }

@@ -137,9 +137,13 @@ __device__ __forceinline__ double inv_root(double m) {
 //    D 4.5^K.
 struct CtrlConsts {
   double accept_sum, lo, hi, scale;
+  // sums below it were taken from scales whose reciprocals are normal numbers: a subnormal scale
+  // makes a sum infinite or NaN, and tolerances that can make one above 2^1022 (whose quotients
+  // come out as 0) leave no sum below
+  double sum_limit;
 };
 
-__host__ inline CtrlConsts make_ctrl_consts(int D, int K) {
+__host__ inline CtrlConsts make_ctrl_consts(int D, int K, double rtol, double atol) {
   const double A = kAcceptMax, dd = (double)D;
   double x = A * dd;  // then walk to the last double whose quotient still rounds to <= A
   while (x / dd > A) x = std::nextafter(x, 0.0);
@@ -149,6 +153,7 @@ __host__ inline CtrlConsts make_ctrl_consts(int D, int K) {
   c.lo = dd * std::pow(0.18, K);
   c.hi = dd * std::pow(4.5, K);
   c.scale = Ctrl::SAFETY * std::pow(dd, 1.0 / K);
+  c.sum_limit = rtol < 0.125 && atol < 1e300 ? INFINITY : -1.0;
   return c;
 }
 
@@ -203,11 +208,14 @@ __device__ __forceinline__ double step_from_sum(double S, double h, const CtrlCo
 // 1 / x without a branch: the hardware's approximate reciprocal (PTX rcp.approx.ftz.f64, about
 // 2^-20 relative) and one third-order step of the residual series (Householder's method:
 // with e = 1 - x r0, 1 / x = r0 (1 + e + e^2 + ...), truncated below 2^-58), within 2 ulp of
-// the quotient.  Where the approximation is 0, infinite, subnormal or NaN (x infinite, 0 or at
-// the ends of the range) it is the result itself, as the quotient is there.  A division
-// carries a branch to its general case, which the instructions after it cannot be scheduled
-// across; the error norm and W's pivots take one to eight reciprocals per attempt on its
-// dependent chain.
+// the quotient where x and 1 / x are normal numbers, and 1 / x where x is 0, infinite or NaN.
+// The approximation flushes to zero, so a subnormal x gives infinity and one above 2^1022 gives
+// 0, where the quotient may be neither: the error norm divides there (norm_failed); a pivot of
+// W can get there only from entries whose products overflow one binary order further on.  A
+// division carries a branch to its general case, which the instructions after it cannot be
+// scheduled across; the error norm and W's pivots take one to eight reciprocals per attempt on
+// its dependent chain (a branch to the division in each: an attempt alone of Van der Pol 0.462
+// / 0.514 us, of HIRES 1.08 / 1.50).
 __device__ __forceinline__ double reciprocal_step(double x, double r0) {
   const double e = fma(-x, r0, 1.0);
   return fma(r0, fma(e, e, e), r0);
@@ -519,6 +527,53 @@ struct RecordArgs {
   CtrlConstsF ctrlf{};  // the float32 route's controller constants (set by its launcher)
 };
 
+// Vectors by value, for functions out of line (no address of a register array is taken).
+template <int N>
+struct DVec {
+  double v[N];
+};
+template <int N>
+__device__ __forceinline__ DVec<N> to_dvec(const double* a) {
+  DVec<N> r;
+#pragma unroll
+  for (int i = 0; i < N; ++i) r.v[i] = a[i];
+  return r;
+}
+template <int N>
+__device__ __forceinline__ void from_dvec(const DVec<N>& r, double* a) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) a[i] = r.v[i];
+}
+
+// The sum of wrms_sumsq with the quotients divided out.
+template <int D>
+__device__ __noinline__ double wrms_divided(DVec<D> e, DVec<D> y, DVec<D> yn, double rtol,
+                                            double atol) {
+  double q[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    const double c = e.v[i] / (atol + rtol * fmax(fabs(y.v[i]), fabs(yn.v[i])));
+    q[i] = c * c;
+  }
+  return wrms_sum<D>(q);
+}
+
+// Whether an attempt's error norm is NaN (dt would turn NaN and the loop could never finish), m
+// being wrms_sumsq's sum.  Where its quotients are products with reciprocals, a sum that is not
+// below CtrlConsts::sum_limit may come from a scale outside reciprocal's range: the sum is then
+// taken again from the quotients.  One branch for both questions, and the divisions out of line
+// (an attempt alone of Van der Pol, Rosenbrock23: no check of the range 0.463 us, this 0.473, a
+// branch of its own 0.496; HIRES 1.08 / 1.10 / 1.13).
+template <int D, bool kShare = true>
+__device__ __forceinline__ bool norm_failed(double& m, const double* e, const double* y,
+                                            const double* yn, const RecordArgs& a) {
+  if constexpr (!(kShare && D >= 2 && D <= 4)) {
+    if (m < a.ctrl.sum_limit) return false;
+    m = wrms_divided<D>(to_dvec<D>(e), to_dvec<D>(y), to_dvec<D>(yn), a.rtol, a.atol);
+  }
+  return !(m == m);
+}
+
 struct AdjointArgs {
   long long n;
   const double* p;
@@ -678,8 +733,8 @@ __device__ __forceinline__ bool tsit5_attempt(const RecordArgs& a, long long j,
   for (int i = 0; i < D; ++i)
     e[i] = h * (T::E1 * k1[i] + T::E2 * S.k2[i] + T::E3 * S.k3[i] + T::E4 * S.k4[i] +
                 T::E5 * S.k5[i] + T::E6 * S.k6[i] + T::E7 * ko[i]);
-  const double m = wrms_sumsq<D>(e, y, yo, a.rtol, a.atol);
-  if (!(m == m)) {  // NaN error: dt would turn NaN and the loop could never finish
+  double m = wrms_sumsq<D>(e, y, yo, a.rtol, a.atol);
+  if (norm_failed<D>(m, e, y, yo, a)) {
     c.st = 1;
     return false;
   }

@@ -98,3 +98,47 @@ def test_reciprocal_matches_division(gslib, cuda):
     n = x.size - edges.size
     assert (np.abs(r[:n] - ref[:n]) <= 2.0 * np.spacing(np.abs(ref[:n]))).all()
     np.testing.assert_array_equal(r[n:], ref[n:])
+
+
+def test_reciprocal_at_the_ends_of_the_range(gslib, cuda):
+    """The hardware's approximation flushes to zero: a subnormal operand gives infinity and one
+    above 2^1022 zero, with its sign (the error norm divides there, test_tiny_scales).  It reads
+    the operand's upper 32 bits, so just above 2^1022 it is still refined."""
+    L = ctypes.CDLL(str(ROOT / "gradsolve_b200" / "libgsprobe.so"))
+    x = np.array([5e-324, 1e-309, 2.2e-308, np.nextafter(np.finfo(np.float64).tiny, 0.0),
+                  np.nextafter(2.0 ** 1022, np.inf), 1e308, np.finfo(np.float64).max])
+    x = np.concatenate([x, -x])
+    xd = torch.tensor(x, device=cuda)
+    r, ref = torch.empty_like(xd), torch.empty_like(xd)
+    P = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    assert L.gs_probe_reciprocal(P(xd), ctypes.c_longlong(x.size), P(r), P(ref), None) == 0
+    r, ref = r.cpu().numpy(), ref.cpu().numpy()
+    edge = np.abs(x) == np.nextafter(2.0 ** 1022, np.inf)
+    assert (np.abs(r[edge] - ref[edge]) <= 2.0 * np.spacing(np.abs(ref[edge]))).all()
+    want = np.copysign(np.where(np.abs(x) < 1.0, np.inf, 0.0), x)
+    np.testing.assert_array_equal(r[~edge], want[~edge])
+
+
+@pytest.mark.parametrize("schedule", ["static", "refill"])
+@pytest.mark.parametrize("method,field", [("tsit5", "linear_1"), ("tsit5", "linear_8"),
+                                          ("tsit5", "linear_32"), ("rosenbrock23", "linear_1"),
+                                          ("rosenbrock23", "linear_3")])
+def test_tiny_scales(gslib, cuda, method, field, schedule):
+    """Without an absolute tolerance a linear field's attempts do not depend on its state's size,
+    subnormal scales of the error included (rtol 0.5: the route for scales above 2^1022)."""
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec = field_spec(field)
+    p = torch.zeros(3, max(spec.nparam, 1), dtype=torch.float64, device=cuda)
+    t1v = None if schedule == "static" else torch.full((3,), 1.0, dtype=torch.float64,
+                                                       device=cuda)
+    for rtol in (1e-6, 0.5):
+        y0 = torch.tensor([[1.0], [1e-303], [3e-304]], dtype=torch.float64,
+                          device=cuda).repeat(1, spec.dim)
+        r = engine.forward_record(method, spec, y0, p, t0=0.0, t1=1.0, t1v=t1v, rtol=rtol,
+                                  atol=0.0, schedule=schedule)
+        assert r.status.tolist() == [0, 0, 0], (rtol, r.status)
+        assert r.n_acc.tolist() == [int(r.n_acc[0])] * 3 and \
+            r.n_rej.tolist() == [int(r.n_rej[0])] * 3
+        scaled = r.y_final / y0
+        assert float((scaled / scaled[0] - 1.0).abs().max()) <= 1e-9
