@@ -290,20 +290,35 @@ def build_replay_state(problem, y0, params, *, method: str, rtol: float, atol: f
     spec, y0_t, p_t, pk = _prepare(problem, y0, params, dev)
     t1s, t1v = _t1_arg(problem, t1, dev)
     ms = int(max_steps or 100000)
-    # ("sqrt" takes its interval from the capacity, so it keeps the default one)
+    # ("sqrt" takes its interval from the capacity, so it keeps the default one; an interval that
+    # forward_record refuses is left to it)
     cap0, budget = engine.DEFAULT_CAP0, None
-    if checkpoint != "sqrt":
+    if checkpoint != "sqrt" and not (isinstance(checkpoint, int) and checkpoint < 1):
         budget = engine._checkpoint_budget()
         K = (checkpoint if isinstance(checkpoint, int) else 1 if checkpoint == "all" else
              engine.tuned_ckpt_every(method, spec, precision) or 2)
         cap0 = engine.first_capacity(y0_t.shape[0], spec.dim, ms, K, precision, budget)
-    r = engine.forward_record(method, spec, y0_t, pk, t0=float(problem.t0), t1=t1s, t1v=t1v,
-                              rtol=rtol, atol=atol, max_steps=ms, cap0=cap0,
-                              checkpoint=checkpoint, budget_bytes=budget, precision=precision,
-                              # the float32 route records without dense output: its closure
-                              # replays the saved states at the recording point
-                              saveat_ts=None if precision == "float32" else saveat)
+
+    def forward(cap0, budget):
+        return engine.forward_record(
+            method, spec, y0_t, pk, t0=float(problem.t0), t1=t1s, t1v=t1v, rtol=rtol, atol=atol,
+            max_steps=ms, cap0=cap0, checkpoint=checkpoint, budget_bytes=budget,
+            precision=precision,
+            # the float32 route records without dense output: its closure replays the saved
+            # states at the recording point
+            saveat_ts=None if precision == "float32" else saveat)
+
+    r = None
+    if cap0 > engine.DEFAULT_CAP0:  # (the budget may be some seconds old, or the memory in pieces)
+        try:
+            r = forward(cap0, budget)
+        except torch.OutOfMemoryError:
+            budget = None
+    if r is None:
+        r = forward(engine.DEFAULT_CAP0, budget)
     engine.raise_on_failed(r, ms, t1s)
+    if budget is not None:
+        r = engine.fit_record(r, budget)
     # queued after the checks' synchronisation, so the sort runs on the device while the host
     # goes on to the closure call and the cotangent; the reverse pass picks it up
     engine.prepare_lane_order(r)
