@@ -1223,13 +1223,15 @@ _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 #   even batches, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
 #   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 392 / 230, 16,384
 #   409 / 667, 262,144 2.08 / 4.94 ms.
-# The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Even
-# Tsit5 batches are split within SPLIT_EVEN_CAP steps of record: over thousands of steps of an
-# expanding flow (Lorenz, t = 70, gradients of 1e20) the two evaluation orders differ by 1e-8.
+# The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Tsit5
+# trajectories are split within SPLIT_TSIT5_STEPS steps taken: over thousands of steps of an
+# expanding flow (Lorenz, t = 70, gradients of 1e21) both evaluation orders are 1e-13 of a row
+# from 80-bit arithmetic, 5e-12 at most, but components that are small beside their row then
+# differ between the two by 1e-8 of themselves.
 SPLIT_MAX_DIM = 3
 SPLIT_EVEN_MAX = {METHOD_TSIT5: 2048, METHOD_ROS23: 8192}
 SPLIT_EVEN_SAVEAT_MAX = 4096
-SPLIT_EVEN_CAP = 4096
+SPLIT_TSIT5_STEPS = 4096
 SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without asking for the budget
 PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
 
@@ -1258,6 +1260,29 @@ def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> b
         return False
     key = (r.method, r.spec.key)  # (a pinned occupancy instance is one thread per trajectory)
     return key not in _OCC_REV or _OCC_REV[key] == _OCC_TUNED.get(key)
+
+
+def _few_steps(r) -> bool:
+    """No trajectory of r takes more than SPLIT_TSIT5_STEPS steps.  The capacity says so, or the
+    step counts: read once per record, with a synchronisation where no check has read them yet
+    (a record whose capacity is max_steps, or a caller's mesh); unread ones do not while a graph
+    is captured."""
+    for _rows, rr in _parts(r):
+        if rr.cap <= SPLIT_TSIT5_STEPS or rr.n == 0:
+            continue
+        if rr.steps_max is None:
+            if torch.cuda.is_current_stream_capturing():
+                return False
+            rr.steps_max = int(rr.n_acc.max().item())
+        if rr.steps_max > SPLIT_TSIT5_STEPS:
+            return False
+    return True
+
+
+def _lanes_for(r, saveat: bool) -> int:
+    """Lanes per trajectory of r's split reverse pass, 0: not split."""
+    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, saveat, r.method)
+    return lanes if lanes and (r.method == METHOD_ROS23 or _few_steps(r)) else 0
 
 
 def _adjoint_split(r: Record, lanes: int, p, ybar, ts, ysbar, want_y0, want_p, order,
@@ -1301,8 +1326,7 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
     nonstiff fields), "recompute" one per thread, and "auto" is "pairs" where it is built."""
     lanes = None
     if _split_applies(r, precision, schedule, variant):
-        if r.uneven or r.method == METHOD_ROS23 or r.cap <= SPLIT_EVEN_CAP:
-            lanes = split_lanes(r.n, r.spec.dim, not r.uneven, False, r.method) or None
+        lanes = _lanes_for(r, False) or None
         if lanes is None and _paired(r):
             lanes = PAIRED
     if schedule == "auto" and r.uneven and precision != "float32":
@@ -1495,8 +1519,8 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
     ``schedule="auto"``, float64, where split_lanes says so: the split reverse pass; else it refills
     lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
     per trajectory for an even one."""
-    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, True)
-    if r.n and lanes and _split_applies(r, precision, schedule):
+    lanes = _lanes_for(r, True) if r.n and _split_applies(r, precision, schedule) else 0
+    if lanes:
         words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
         if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
             f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
