@@ -18,7 +18,6 @@ import copy
 import ctypes
 import math
 import threading
-import weakref
 from dataclasses import dataclass
 from typing import Optional
 
@@ -152,44 +151,61 @@ def first_capacity(n: int, dim: int, max_steps: int, ckpt_every: int, precision:
     return max(lo, min(int(max_steps), cap))
 
 
-# What a record of a first capacity holds beyond the steps its batch took lives as long as its
-# closure, so fit_record bounds it: the records alive on a device hold at most the share of the
-# budget that one first capacity may take beyond their steps, all together, and a record whose
-# excess would pass that is copied into buffers of its steps' size.  (Copying at once would cost
-# a closure of a thousand Robertson trajectories 480 -> 550 us, and HIRES 8192 0.23 of 4.0 ms.)
-_SLACK: dict = {}  # device index -> bytes that the records alive hold beyond their steps
-_SLACK_LOCK = threading.RLock()  # (a record may be collected while its thread holds it)
+# What a record of a first capacity holds beyond DEFAULT_CAP0 steps lives as long as its closure,
+# so fit_record bounds it: the records alive on a device hold at most the share of the budget
+# that one first capacity may take, all together, and one whose excess would pass that is
+# copied into buffers of its steps' size.  (Copying at once would cost a closure of a thousand
+# Robertson trajectories 480 -> 550 us, and HIRES 8192 0.23 of 4.0 ms.)
+_EXCESS: dict = {}  # device index -> bytes
+_EXCESS_LOCK = threading.RLock()  # (a record may be collected while its thread holds it)
 
 
-def _add_slack(index, nbytes: int) -> None:
-    with _SLACK_LOCK:
-        _SLACK[index] = _SLACK.get(index, 0) + nbytes
+class _Excess:
+    """Bytes counted in _EXCESS while the object lives."""
+
+    def __init__(self, index, nbytes: int):
+        self.index, self.nbytes = index, nbytes
+        _EXCESS[index] = _EXCESS.get(index, 0) + nbytes
+
+    def __del__(self):
+        with _EXCESS_LOCK:
+            _EXCESS[self.index] -= self.nbytes
+
+
+def _record_size(r, cap: int) -> tuple:
+    """Elements of a record of r's batch and type with capacity cap: dts, checkpoints."""
+    width, ctrl = ((ckpt_width_f32(r.spec.dim), 2 * CTRL_DOUBLES) if r.rec.element_size() == 4
+                   else (ckpt_width(r.spec.dim), CTRL_DOUBLES))
+    return (r.n * -(-cap // 4) * 4,
+            _lib.lib().gs_ckpt_slots(cap, r.ckpt_every) * r.n * width + ctrl)
+
+
+def longest_steps(r) -> int:
+    """Steps of the longest trajectory of a Record (one synchronisation, the first time)."""
+    if r.steps_max is None:
+        r.steps_max = int(r.n_acc.max().item()) if r.n else 0
+    return r.steps_max
 
 
 def fit_record(r, budget_bytes: int):
-    """The record itself, or a copy of capacity r.steps_max (its unwritten slots given back)."""
-    if not isinstance(r, Record) or r.steps_max is None or r.n == 0:
+    """The record itself, or a copy of its longest trajectory's capacity."""
+    if not isinstance(r, Record) or r.cap <= DEFAULT_CAP0 or r.n == 0:
         return r
-    cap = max(4, -(-r.steps_max // 4) * 4)
+    excess = r.nbytes - sum(_record_size(r, DEFAULT_CAP0)) * r.rec.element_size()
+    index = r.rec.device.index
+    with _EXCESS_LOCK:
+        if _EXCESS.get(index, 0) + excess <= budget_bytes // CAP_SHARE:
+            r.excess = _Excess(index, excess)
+            return r
+    cap = max(4, -(-longest_steps(r) // 4) * 4)
     if cap >= r.cap:
         return r
-    word = r.rec.element_size()
-    width, ctrl = ((ckpt_width_f32(r.spec.dim), 2 * CTRL_DOUBLES) if word == 4 else
-                   (ckpt_width(r.spec.dim), CTRL_DOUBLES))
-    rows = _lib.lib().gs_ckpt_slots(cap, r.ckpt_every) * r.n * width
-    used = (r.n * cap + rows + ctrl) * word
-    slack, index = r.nbytes - used, r.rec.device.index
-    with _SLACK_LOCK:
-        if _SLACK.get(index, 0) + slack <= budget_bytes // CAP_SHARE:
-            _add_slack(index, slack)
-            weakref.finalize(r, _add_slack, index, -slack).atexit = False
-            return r
     # step-major chunks and slots: a record of fewer steps is the start of a longer one (what
     # stands in the control block after the checkpoints is zeroed by its users)
+    rec, ckpt = _record_size(r, cap)
     f = copy.copy(r)
     try:
-        f.rec = r.rec[:r.n * cap].clone()
-        f.ckpt = r.ckpt[:rows + ctrl].clone()
+        f.rec, f.ckpt = r.rec[:rec].clone(), r.ckpt[:ckpt].clone()
     except torch.OutOfMemoryError:
         return r
     f.cap = cap
@@ -301,8 +317,8 @@ class Record:
     ys: Optional[torch.Tensor] = None  # (n, K, D) dense output of the forward, if asked for
     lane_order: Optional[torch.Tensor] = None  # the reverse pass's lane order, if prepared
     status_max: Optional[int] = None  # largest status code, once a check has read it
-    counts: Optional[torch.Tensor] = None  # (3, n): n_acc, n_rej, status, where they are one block
-    steps_max: Optional[int] = None  # largest step count, once a check has read it
+    steps_max: Optional[int] = None  # largest step count, once read (longest_steps)
+    excess: object = None    # what fit_record counts of this record while it lives
 
     @property
     def nbytes(self) -> int:
@@ -508,20 +524,6 @@ def _status_max(status: torch.Tensor, device) -> int:
     if vals[1] != 0:
         _raise_bad_moves(c, int(vals[1]))
     return int(vals[0])
-
-
-def _read_counts(r: Record) -> None:
-    """Fill r.status_max and, where the forward's counts are one block, r.steps_max: one
-    reduction and the forward's one synchronisation."""
-    if r.counts is None:
-        r.status_max = _status_max(r.status, r.status.device)
-        return
-    top = r.counts.amax(dim=1)
-    c = _BAD_MOVES.get(r.counts.device.index)
-    vals = (top if c is None else torch.cat([top.to(torch.int64), c])).tolist()
-    if c is not None and vals[3] != 0:
-        _raise_bad_moves(c, int(vals[3]))
-    r.steps_max, r.status_max = int(vals[0]), int(vals[2])
 
 
 def _movable(t: torch.Tensor) -> bool:
@@ -987,8 +989,9 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False
             tuned = min(tuned or SAVEAT_CKPT_MAX, SAVEAT_CKPT_MAX)
         K = choose_ckpt_every(kw["checkpoint"], spec.dim, n, cap, kw["budget_bytes"], tuned)
     yf = ws.y_final if ok else torch.empty_like(y0)
-    counts = ws.counts if ok else torch.empty((3, n), dtype=torch.int32, device=device)
-    n_acc, n_rej, status = (ws.n_acc, ws.n_rej, ws.status) if ok else counts.unbind(0)
+    n_acc, n_rej, status = ((ws.n_acc, ws.n_rej, ws.status) if ok else
+                            tuple(torch.empty(n, dtype=torch.int32, device=device)
+                                  for _ in range(3)))
     if (ok and ws.cap == cap and ws.ckpt_every == K and ws.rec.numel() > 2 and
             ws.rec.dtype == record_dtype(precision)):
         rec, ckpt = ws.rec, ws.ckpt
@@ -1021,7 +1024,7 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False
         ys = torch.empty((0, _ts_arg(saveat_ts, 0)[2] if saveat_ts.ndim == 1 else
                           saveat_ts.shape[1], spec.dim), dtype=torch.float64, device=device)
     return Record(method, spec, n, float(kw["t0"]), cap, K, rec, ckpt, yf, n_acc, n_rej,
-                  status, uneven=t1v is not None, ys=ys, counts=counts)
+                  status, uneven=t1v is not None, ys=ys)
 
 
 def _assemble(method, spec, n, device, parts, t1v, saveat_ts, streams, sub=None):
@@ -1058,7 +1061,7 @@ def _grow(method, spec, y0, p, t1v, saveat_ts, r0, streams, kw):
     max_steps = int(kw["max_steps"])
     if n == 0 or r0.cap >= max_steps:
         return r0
-    _read_counts(r0)
+    r0.status_max = _status_max(r0.status, y0.device)
     if r0.status_max < 3:  # no row overflowed the record
         return r0
     rows = torch.nonzero(r0.status == 3).squeeze(1)
@@ -1146,10 +1149,7 @@ def raise_on_failed(r: Record, max_steps: int, t1) -> None:
     if r.n == 0:
         return
     if r.status_max is None:  # (a record of max_steps capacity: the forward read no status)
-        if isinstance(r, Record):
-            _read_counts(r)
-        else:
-            r.status_max = _status_max(r.status, r.status.device)
+        r.status_max = _status_max(r.status, r.status.device)
     if r.status_max == 0:
         return
     bad = torch.nonzero(r.status != 0).flatten()
@@ -1263,18 +1263,14 @@ def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> b
 
 
 def _few_steps(r) -> bool:
-    """No trajectory of r takes more than SPLIT_TSIT5_STEPS steps.  The capacity says so, or the
-    step counts: read once per record, with a synchronisation where no check has read them yet
-    (a record whose capacity is max_steps, or a caller's mesh); unread ones do not while a graph
-    is captured."""
+    """No trajectory of r takes more than SPLIT_TSIT5_STEPS steps: the capacity says so, or the step
+    counts, read once per record (not while a graph is captured)."""
     for _rows, rr in _parts(r):
         if rr.cap <= SPLIT_TSIT5_STEPS or rr.n == 0:
             continue
-        if rr.steps_max is None:
-            if torch.cuda.is_current_stream_capturing():
-                return False
-            rr.steps_max = int(rr.n_acc.max().item())
-        if rr.steps_max > SPLIT_TSIT5_STEPS:
+        if rr.steps_max is None and torch.cuda.is_current_stream_capturing():
+            return False
+        if longest_steps(rr) > SPLIT_TSIT5_STEPS:
             return False
     return True
 

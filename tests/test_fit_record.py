@@ -19,18 +19,17 @@ def _record(n, cap, steps, K=2, precision="float64"):
     ckpt.copy_(-torch.arange(ckpt.numel()).to(ckpt.dtype))
     acc = torch.full((n,), steps, dtype=torch.int32)
     return engine.Record("tsit5", field_spec("lorenz"), n, 0.0, cap, K, rec, ckpt,
-                         torch.zeros(n, 3, dtype=torch.float64), acc, acc * 0, acc * 0,
-                         steps_max=steps)
+                         torch.zeros(n, 3, dtype=torch.float64), acc, acc * 0, acc * 0)
 
 
 @pytest.mark.parametrize("precision", ["float64", "float32"])
-@pytest.mark.parametrize("steps", [0, 1, 7, 8, 95])
+@pytest.mark.parametrize("steps", [0, 1, 7, 8, 95, 1500, 2048])
 @pytest.mark.parametrize("K", [1, 2, 5])
 def test_copy_is_the_start_of_the_record(gslib, K, steps, precision):
-    r = _record(3, 96, steps, K, precision)
+    r = _record(3, 2048, steps, K, precision)
     f = engine.fit_record(r, 0)  # no share at all: every excess is copied away
     cap = max(4, -(-steps // 4) * 4)
-    if cap >= 96:
+    if cap >= 2048:
         assert f is r
         return
     assert f.cap == cap and f.n_acc is r.n_acc and f.ckpt_every == K
@@ -43,19 +42,25 @@ def test_copy_is_the_start_of_the_record(gslib, K, steps, precision):
     assert torch.equal(f.ckpt[:rows], r.ckpt[:rows])
 
 
+def test_default_records_are_not_counted(gslib, monkeypatch):
+    monkeypatch.setattr(engine, "_EXCESS", {})
+    r = _record(3, engine.DEFAULT_CAP0, 7)
+    assert engine.fit_record(r, 0) is r and engine._EXCESS == {}
+
+
 def test_excess_is_bounded_over_the_records_alive(gslib, monkeypatch):
-    monkeypatch.setattr(engine, "_SLACK", {})
-    r = _record(64, 4096, 2048)
-    excess = r.nbytes - _record(64, 2048, 2048).nbytes
+    monkeypatch.setattr(engine, "_EXCESS", {})
+    r = _record(64, 4096, 1500)
+    excess = r.nbytes - _record(64, engine.DEFAULT_CAP0, 0).nbytes
     budget = engine.CAP_SHARE * (excess + excess // 2)  # room for one record's excess, not two
     assert engine.fit_record(r, budget) is r
-    assert engine._SLACK[None] == excess
-    other = _record(64, 4096, 2048)
+    assert engine._EXCESS[None] == excess
+    other = _record(64, 4096, 1500)
     fitted = engine.fit_record(other, budget)
-    assert fitted is not other and fitted.cap == 2048
+    assert fitted is not other and fitted.cap == 1500 and engine._EXCESS[None] == excess
     del r
     gc.collect()
-    assert engine._SLACK[None] == 0
+    assert engine._EXCESS[None] == 0
     assert engine.fit_record(other, budget) is other
 
 
@@ -77,7 +82,7 @@ def _gradient(f, y0, p):
 @pytest.mark.gpu
 def test_closures_alive_share_one_excess(gslib, cuda, monkeypatch):
     import gradsolve_b200 as gs
-    monkeypatch.setattr(engine, "_SLACK", {})
+    monkeypatch.setattr(engine, "_EXCESS", {})
     monkeypatch.setattr(engine, "_checkpoint_budget", lambda: 8 << 30)
     problem, y0, p = _robertson(1000, cuda)
     kw = dict(wrt=("y0", "params"), rtol=1e-6, atol=1e-10)
@@ -93,7 +98,7 @@ def test_closures_alive_share_one_excess(gslib, cuda, monkeypatch):
             assert torch.equal(a, b)
     del alive, f
     gc.collect()
-    assert engine._SLACK[0] == 0
+    assert engine._EXCESS[0] == 0
 
 
 @pytest.mark.gpu
