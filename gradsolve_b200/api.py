@@ -296,7 +296,7 @@ def build_replay_state(problem, y0, params, *, method: str, rtol: float, atol: f
     if checkpoint != "sqrt" and not (isinstance(checkpoint, int) and checkpoint < 1):
         budget = engine._checkpoint_budget()
         K = (checkpoint if isinstance(checkpoint, int) else 1 if checkpoint == "all" else
-             engine.tuned_ckpt_every(method, spec, precision) or 2)
+             engine.auto_ckpt_every(method, spec, y0_t.shape[0], precision, t1v, saveat) or 2)
         cap0 = engine.first_capacity(y0_t.shape[0], spec.dim, ms, K, precision, budget)
 
     def forward(cap0, budget):

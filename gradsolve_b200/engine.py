@@ -245,6 +245,18 @@ def tuned_ckpt_every(method: str, spec: FieldSpec, precision: str) -> Optional[i
     return _TUNED.get((method, spec.key, precision))
 
 
+def auto_ckpt_every(method: str, spec: FieldSpec, n: int, precision: str, t1v,
+                    saveat_ts) -> Optional[int]:
+    """The interval checkpoint="auto" starts from (choose_ckpt_every's ``tuned``)."""
+    tuned = tuned_ckpt_every(method, spec, precision)
+    if precision != "float64":
+        return tuned
+    if tuned is None or _pairs(spec.dim, n, t1v, saveat_ts, precision):
+        tuned = 2  # (a small batch: its checkpoints are no matter)
+    # (dense output walks K / 2 steps from a checkpoint per requested time)
+    return tuned if saveat_ts is None else min(tuned, SAVEAT_CKPT_MAX)
+
+
 @_tuner
 def autotune_ckpt_every(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tensor, *,
                         t0: float, t1: float, rtol: float, atol: float,
@@ -264,6 +276,9 @@ def autotune_ckpt_every(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch
         candidates = TUNE_CANDIDATES_F32 if precision == "float32" else TUNE_CANDIDATES
     budget = _checkpoint_budget()
     row = 4 * ckpt_width_f32(spec.dim) if precision == "float32" else 8 * ckpt_width(spec.dim)
+    # the one-thread passes, whatever pass a batch of the sample's size takes: the choice is kept
+    # for every size
+    sched = "auto" if precision != "float64" else "static" if tv is None else "refill"
     times = {}
     for K in candidates:
         if (DEFAULT_CAP0 // K + 2) * m * row > budget and K != candidates[-1]:
@@ -272,18 +287,18 @@ def autotune_ckpt_every(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch
                   checkpoint=K, precision=precision)
         r = forward_record(method, spec, ys, ps, **kw)
         ybar = torch.ones_like(r.y_final)
-        adjoint(r, ps, ybar, precision=precision)  # warm
+        adjoint(r, ps, ybar, precision=precision, schedule=sched)  # warm
         for _ in range(2):  # the steady state of a reused workspace (lanes ordered by cost,
             # the allocator's blocks cycling between two steps' outputs): no cudaMalloc timed
             r = forward_record(method, spec, ys, ps, workspace=r, **kw)
-            adjoint(r, ps, ybar, precision=precision)
+            adjoint(r, ps, ybar, precision=precision, schedule=sched)
         # forward (checkpoint writes grow as K shrinks) + reverse pass, buffers reused
         ms = float("inf")
         for _ in range(reps):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
             r = forward_record(method, spec, ys, ps, workspace=r, **kw)
-            adjoint(r, ps, ybar, precision=precision)
+            adjoint(r, ps, ybar, precision=precision, schedule=sched)
             e1.record()
             e1.synchronize()
             ms = min(ms, e0.elapsed_time(e1))
@@ -800,10 +815,11 @@ def autotune_occupancy(spec: FieldSpec, y0: torch.Tensor, p: torch.Tensor, *, t0
     if all(rr.ckpt_every == 2 for rr in parts) and len(rev) > 1:
         ybar = torch.ones_like(r.y_final)
         times = {}
-        for b in rev:
+        sched = "refill" if r.uneven else "static"  # (the instances, not the passes of small
+        for b in rev:                               # batches)
             _OCC_REV[key] = b
-            adjoint(r, ps, ybar)  # warm
-            times[b] = _time_ms(lambda: adjoint(r, ps, ybar), reps)
+            adjoint(r, ps, ybar, schedule=sched)  # warm
+            times[b] = _time_ms(lambda: adjoint(r, ps, ybar, schedule=sched), reps)
         _OCC_REV[key] = _pick(times)
     _OCC_TUNED[key] = _OCC_REV[key]
     return _OCC[key], _OCC_REV[key]
@@ -915,7 +931,8 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
             precision == "float64"):
         autotune_lanes(spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                        max_steps=max_steps)
-    if checkpoint == "auto" and tuned_ckpt_every(method, spec, precision) is None and n >= 4096:
+    if (checkpoint == "auto" and tuned_ckpt_every(method, spec, precision) is None and
+            n >= 4096 and not _pairs(spec.dim, n, t1v, saveat_ts, precision)):
         autotune_ckpt_every(method, spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                             max_steps=max_steps, precision=precision)
     occ_sched = "static" if method == METHOD_ROS23 and schedule == "auto" and isinstance(
@@ -981,12 +998,7 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False
     if kw["checkpoint"] == "auto" and ok and ws.cap == cap and ws.rec.numel() > 2:
         K = ws.ckpt_every  # sticky: the workspace's interval, so its buffers are reused
     else:
-        tuned = tuned_ckpt_every(method, spec, precision)
-        if tuned is None and precision == "float64":
-            tuned = 2  # (a batch too small to tune on: its checkpoints are no matter)
-        if saveat_ts is not None and precision == "float64":
-            # (dense output walks K / 2 steps from a checkpoint per requested time)
-            tuned = min(tuned or SAVEAT_CKPT_MAX, SAVEAT_CKPT_MAX)
+        tuned = auto_ckpt_every(method, spec, n, precision, t1v, saveat_ts)
         K = choose_ckpt_every(kw["checkpoint"], spec.dim, n, cap, kw["budget_bytes"], tuned)
     yf = ws.y_final if ok else torch.empty_like(y0)
     n_acc, n_rej, status = ((ws.n_acc, ws.n_rej, ws.status) if ok else
@@ -1248,10 +1260,17 @@ def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD
     return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
 
 
+def _pairs(dim: int, n: int, t1v, saveat_ts, precision: str) -> bool:
+    """Batches of the sizes that two warps per 32 trajectories are for: they take the interval that
+    pass is built for, K = 2, and not the one tuned on larger ones."""
+    most = 1 << 14 if dim <= 4 else 1 << 13 if dim <= 8 else 0
+    return 0 < n <= most and t1v is None and saveat_ts is None and precision == "float64"
+
+
 def _paired(r) -> bool:
     """Two warps per 32 trajectories: even batches whose blocks are all resident, short segments."""
-    most = 1 << 14 if r.spec.dim <= 4 else 1 << 13 if r.spec.dim <= 8 else 0
-    return 0 < r.n <= most and not r.uneven and all(rr.ckpt_every <= 2 for _rows, rr in _parts(r))
+    return (not r.uneven and _pairs(r.spec.dim, r.n, None, None, "float64") and
+            all(rr.ckpt_every <= 2 for _rows, rr in _parts(r)))
 
 
 def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> bool:
