@@ -1769,39 +1769,7 @@ int launch_saveat_states(const gs::RecordArgs& a, cudaStream_t s) {
   gs::saveat_states_kernel<F, M><<<grid_for(a.n * parts), kBlock, 0, s>>>(b);
   return cuda_check("saveat_states_kernel");
 }
-// The pass of its own walks K / 2 steps from a checkpoint to a requested time where the forward
-// has the state at hand, so it loses where those steps cost more than the lanes that wait: long
-// intervals, and batches that fill the chip.  B200, forward with its 64 times, in the forward /
-// apart, us, at K = 2, 8, 32:
-//   one end time: Lorenz 4096 171 / 144, 169 / 149, 167 / 161   8192 175 / 152, 170 / 157, 171 / 185
-//               16,384 177 / 173, 177 / 188, 180 / 237   262,144 906 / 999, 782 / 1242, 762 / 1992
-//   Lotka-Volterra 16,384 178 / 146, 177 / 159, 171 / 197   65,536 254 / 273, 262 / 297, 255 / 451
-//   Lorenz-96 of 8 2048 228 / 159, 229 / 167, 224 / 187   8192 231 / 195, 230 / 220, 231 / 281
-//               16,384 250 / 258, 250 / 287, 245 / 425
-//   Robertson 16,384 448 / 337, 438 / 334, 432 / 423   262,144 2321 / 2118, 2277 / 2238, 2248 / 3431
-//   HIRES 1024 701 / 652, 688 / 650, 692 / 693   4096 714 / 693, 702 / 701, 701 / 801
-//               8192 715 / 768, 705 / 777, 702 / 955
-//   per-trajectory end times (lanes refilled, each re-step at its own attempt): Van der Pol 100,000
-//               1449 / 1126, 1435 / 1129, 1372 / 1277   524,288 3383 / 2706, 3353 / 2746, 3321 / 3494
-//   Lorenz 32,768 334 / 220, 316 / 240, 317 / 335   262,144 1107 / 993, 1096 / 1179, 1095 / 1894
-//   Lorenz-96 of 8 8192 333 / 184, 331 / 200, 334 / 266   32,768 457 / 370, 458 / 417, 455 / 633
-//               262,144 2673 / 1944, 2660 / 2323, 2657 / 3863
-//   Robertson 32,768 648 / 426, 641 / 436, 633 / 595   131,072 1399 / 1237, 1360 / 1294, 1341 / 1882
-//   HIRES 8192 1113 / 802, 1087 / 804, 1071 / 1009   32,768 1363 / 1348, 1331 / 1464, 1316 / 2196
-template <class F>
-bool states_apart(const gs::RecordArgs& a, bool stiff) {
-  if (!a.ys || !a.rec || !a.ckpt) return false;
-  constexpr bool small = F::D <= 3;
-  const bool close = a.ck_every <= 8;
-  const long long n = a.n, nk = a.n * a.ck_every;
-  if (a.t1v) {
-    if (small) return close || nk <= (1 << 20);
-    return stiff ? n <= (1 << 13) || nk <= (1 << 16) : close || nk <= (1 << 18);
-  }
-  if (small && stiff) return close || nk <= (1 << 19);
-  if (small) return n <= (1 << 14) && nk <= (1 << 16);
-  return stiff ? n <= (1 << 12) && nk <= (1 << 15) : n <= (1 << 13) && nk <= (1 << 16);
-}
+bool states_apart(const gs::RecordArgs& a) { return a.ys && a.rec && a.ckpt; }
 
 template <class F>
 int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed, FwdLanes lanes,
@@ -1810,8 +1778,7 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
     return coop_refuse<F>("the dense output (saveat)");
   } else {
     if (mixed) return launch_fwd_lanes<F, gs::LaneTsit5Mixed<F>>(a, s, lanes);
-    if (!states_apart<F>(a, false))
-      return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
+    if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
     gs::RecordArgs b = a;
     b.ys = nullptr;
     const int sched = lanes == kStatic ? GS_SCHED_STATIC
@@ -1824,7 +1791,7 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
 template <class F>
 int launch_fwd_saveat_ros23(const gs::RecordArgs& a, cudaStream_t s, FwdLanes lanes,
                             int precision) {
-  if (!states_apart<F>(a, true)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
+  if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
   gs::RecordArgs b = a;
   b.ys = nullptr;
   const int sched = lanes == kStatic ? GS_SCHED_STATIC
@@ -1874,43 +1841,6 @@ int launch_adjoint_paired(const gs::SaveatArgs& a, cudaStream_t s, const long lo
                     order};
   gs::adjoint_paired_kernel<F, S><<<(unsigned)((a.n + 31) / 32), 64, smem, s>>>(b);
   return cuda_check("adjoint_paired_kernel");
-}
-
-// Trajectories that are resident at once with two warps per 32 of them; 0 where that pass is not
-// built or does not fit.  A dense W of more than 3 components (pivoted LU) takes it at K = 2
-// alone: at K = 1 one thread per trajectory is faster at every size (8 components 1756 / 2348 us
-// at 2048), and 128,000 bytes a block leave one per SM (K = 2: 4096 2362 / 2180 us, 4736 2524 /
-// 2604, 8192 2369 / 4450).
-template <class F, class S>
-int paired_room(int K, bool dense_w, long long* room) {
-  const int sd = gs::paired_smem_doubles<F, S>(K);
-  const size_t smem = (size_t)sd * 64 * sizeof(double);
-  *room = 0;
-  if (smem > kSegBudget || (dense_w && K == 1)) return GS_OK;
-  int rc, dev = 0, sms = 0, per_sm = 0;
-  if ((rc = allow_smem(gs::adjoint_paired_kernel<F, S>, smem))) return rc;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs::adjoint_paired_kernel<F, S>, 64,
-                                                      smem);
-  if (e != cudaSuccess)
-    return fail(GS_ERR_CUDA, std::string("CUDA: occupancy query: ") + cudaGetErrorString(e));
-  *room = 32ll * per_sm * sms;
-  return GS_OK;
-}
-template <class F>
-int paired_room_tsit5(int K, long long* room) {
-  if constexpr (F::D <= 8) return paired_room<F, gs::Tsit5Pair<F>>(K, false, room);
-  *room = 0;
-  return GS_OK;
-}
-template <class F>
-int paired_room_ros23(int K, long long* room) {
-  if constexpr (F::D <= 8)
-    return paired_room<F, gs::Ros23Pair<F>>(K, gs::Ros23Pair<F>::kPiv > 0, room);
-  *room = 0;
-  return GS_OK;
 }
 
 template <class F>
@@ -2061,20 +1991,6 @@ extern "C" int gs_adjoint_split(int method, int field, int precision, long long 
   }
   if (method == GS_METHOD_ROS23) {
     GS_ROS23_DISPATCH(field, launch_split_ros23, a, s, lanes, work, order)
-  }
-  return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
-}
-
-extern "C" int gs_adjoint_paired_room(int method, int field, int ckpt_every, long long* room) {
-  const char* who = "gs_adjoint_paired_room";
-  if (!room || ckpt_every < 1 || ckpt_every > gs::KMAX)
-    return fail(GS_ERR_ARG, std::string(who) + ": room and an interval in [1, " +
-                                std::to_string(gs::KMAX) + "] are required");
-  if (method == GS_METHOD_TSIT5) {
-    GS_TSIT5_DISPATCH(field, paired_room_tsit5, ckpt_every, room)
-  }
-  if (method == GS_METHOD_ROS23) {
-    GS_ROS23_DISPATCH(field, paired_room_ros23, ckpt_every, room)
   }
   return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
 }

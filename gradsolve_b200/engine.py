@@ -245,20 +245,13 @@ def tuned_ckpt_every(method: str, spec: FieldSpec, precision: str) -> Optional[i
     return _TUNED.get((method, spec.key, precision))
 
 
-def _own_interval(method: str, spec: FieldSpec, n: int, precision: str, t1v, saveat_ts) -> bool:
-    """Batches whose reverse pass runs two warps per 32 trajectories take the interval it is built
-    for, 2, and not the one tuned on larger ones."""
-    return (precision == "float64" and t1v is None and saveat_ts is None and
-            _pairs(method, spec, n))
-
-
 def auto_ckpt_every(method: str, spec: FieldSpec, n: int, precision: str, t1v,
                     saveat_ts) -> Optional[int]:
     """The interval checkpoint="auto" starts from (choose_ckpt_every's ``tuned``)."""
     tuned = tuned_ckpt_every(method, spec, precision)
     if precision != "float64":
         return tuned
-    if tuned is None or _own_interval(method, spec, n, precision, t1v, saveat_ts):
+    if tuned is None or _pairs(spec.dim, n, t1v, saveat_ts, precision):
         tuned = 2  # (a small batch: its checkpoints are no matter)
     # (dense output walks K / 2 steps from a checkpoint per requested time)
     return tuned if saveat_ts is None else min(tuned, SAVEAT_CKPT_MAX)
@@ -939,7 +932,7 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
         autotune_lanes(spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                        max_steps=max_steps)
     if (checkpoint == "auto" and tuned_ckpt_every(method, spec, precision) is None and
-            n >= 4096 and not _own_interval(method, spec, n, precision, t1v, saveat_ts)):
+            n >= 4096 and not _pairs(spec.dim, n, t1v, saveat_ts, precision)):
         autotune_ckpt_every(method, spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                             max_steps=max_steps, precision=precision)
     occ_sched = "static" if method == METHOD_ROS23 and schedule == "auto" and isinstance(
@@ -971,12 +964,9 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
 
 # Fresh batches from these sizes up run the compacting forward (gs_fwd_record_compact,
 # csrc/gs_compact.cuh): their step counts are not known yet, and where they spread a third of the
-# one-launch forward's lanes idle.  Below, its launches' tails cost what it saves, us, one launch /
-# compacting: Rosenbrock23 Robertson 32,768 278 / 332, 65,536 463 / 477, 131,072 732 / 701, 2^18
-# 1388 / 1247; Van der Pol (stiff, a few long trajectories) 65,536 1097 / 1352, 131,072 2057 / 2172,
-# 2^18 3545 / 3575; Tsit5 Lotka-Volterra 131,072 256 / 262, 2^18 433 / 398; Van der Pol 131,072 303 /
-# 308, 2^18 551 / 500, 2^19 1049 / 865; Lorenz 2^18 1318 / 1294.
-COMPACT_MIN = {METHOD_TSIT5: 1 << 18, METHOD_ROS23: 1 << 17}
+# one-launch forward's lanes idle.  Below, its launches' tails cost what it saves: Robertson 65,536
+# 1.06 / 1.00 ms, Lotka-Volterra (float32 stages) 65,536 137 / 164 us, 2^18 388 / 374 us.
+COMPACT_MIN = {METHOD_TSIT5: 1 << 18, METHOD_ROS23: 1 << 16}
 COMPACT_MAX_DIM = 4
 
 
@@ -988,7 +978,7 @@ def _compacts(method, spec, n, precision, schedule, t1v, saveat_ts) -> bool:
 
 
 def _compact_work(L, code, n, device) -> Optional[torch.Tensor]:
-    """Scratch of the compacting forward, 28 to 88 bytes a trajectory; None where it does not
+    """Scratch of the compacting forward, 30 to 80 bytes a trajectory; None where it does not
     fit (the one-launch forward needs none)."""
     size = L.gs_fwd_compact_bytes(*code, n)
     try:
@@ -1236,19 +1226,15 @@ _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 # takes one, for a chain shorter by the number of lanes), or two warps per 32 trajectories
 # (csrc/gs_paired.cuh, up to 8 components: the one-thread arithmetic).  B200, reverse pass one
 # thread per trajectory / split / two warps:
-#   one end time: Lorenz (t = 1, 112 steps) n = 1024 68 / 25 us, 4096 68 / 39, 8192 48 / - / 29,
-#   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 185 / 43 / 134 us, 4096 191 / 99 / 138,
-#   8192 193 / 161 / 139; Van der Pol (Rosenbrock23, counts spread) 8192 606 / 191 / 524; HIRES
-#   8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
-#   per-trajectory end times (lanes refilled / split): Van der Pol 20,000 463 / 66 us, 65,536 701 /
-#   152, 131,072 784 / 279; with 64 saved times 100,000 1.37 / 0.67 ms (4 lanes), 200,000 1.73 / 1.15,
-#   350,000 1.66 / 2.01, 700,000 2.60 / 3.57;
-#   stiff Van der Pol (8 lanes, K = 2) in batch order 65,536 8.99 / 8.50 ms, 100,000 12.8 / 12.6, 131,072
-#   17.2 / 16.7; planned 131,072 8.7 / 6.6; with 64 saved times in batch order 65,536 11.3 / 9.4,
-#   100,000 14.6 / 14.8, 131,072 15.4 / 19.5; planned 100,000 11.2 / 7.3, 131,072 11.6 / 9.7;
-#   one end time, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
-#   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 483 / 181, 8192 480 / 347;
-#   Van der Pol (Rosenbrock23) 4096 978 / 175.
+#   even batches: Lorenz (t = 1, 112 steps) n = 1024 68 / 25 us, 4096 68 / 39, 8192 48 / - / 29,
+#   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 442 / 45 us, 8192 449 / 197 / 326,
+#   16,384 452 / - / 385; HIRES 8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
+#   per-trajectory end times, 64 saved times: stiff Van der Pol 20,011 9.7 / 1.0 ms (16 lanes),
+#   200,000 11.8 / 9.9, 350,000 11.8 / 20.1; Van der Pol 100,000 1.37 / 0.67 ms (4), 200,000
+#   1.73 / 1.15, 350,000 1.66 / 2.01, 700,000 2.60 / 3.57 (one thread: lanes refilled);
+#   even batches, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
+#   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 392 / 230, 16,384
+#   409 / 667, 262,144 2.08 / 4.94 ms.
 # The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Tsit5
 # trajectories are split within SPLIT_TSIT5_STEPS steps taken: over thousands of steps of an
 # expanding flow (Lorenz, t = 70, gradients of 1e21) both evaluation orders are 1e-13 of a row
@@ -1262,8 +1248,7 @@ SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without askin
 PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
 
 
-def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5,
-                planned: bool = False) -> int:
+def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5) -> int:
     """Lanes per trajectory of the split reverse pass, 0: not split."""
     if even:
         most = SPLIT_EVEN_SAVEAT_MAX if saveat else SPLIT_EVEN_MAX[method]
@@ -1271,40 +1256,21 @@ def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD
         most = 1 << (18 if saveat else 17)
     if dim > SPLIT_MAX_DIM or n > most:
         return 0
-    room = ((1 << 17 if ros else 1 << 16) if even and not saveat else 1 << 19) // max(n, 1)
-    least = 8 if ros and not even else 1
-    return max(least, min(32, 1 << (room.bit_length() - 1) if room else 1))
+    room = (1 << 16 if even and not saveat else 1 << 19) // max(n, 1)
+    return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
 
 
-    ros = method == METHOD_ROS23
 def _pairs(dim: int, n: int, t1v, saveat_ts, precision: str) -> bool:
     """Batches of the sizes that two warps per 32 trajectories are for: they take the interval that
-    elif ros:
-        most = 1 << 17 if planned else 3 << 15
     pass is built for, K = 2, and not the one tuned on larger ones."""
     most = 1 << 14 if dim <= 4 else 1 << 13 if dim <= 8 else 0
     return 0 < n <= most and t1v is None and saveat_ts is None and precision == "float64"
 
 
 def _paired(r) -> bool:
-    """r's reverse pass runs two warps per 32 trajectories."""
-    return not r.uneven and all(_pairs(r.method, r.spec, r.n, rr.ckpt_every)
-                                for _rows, rr in _parts(r))
-
-
-_PAIR_ROOM: dict = {}  # (method, field key, interval, device) -> gs_adjoint_paired_room
-
-
-def _pair_room(method: str, spec: FieldSpec, K: int) -> int:
-    if not torch.cuda.is_initialized():
-        return 0
-    key = (method, spec.key, K, torch.cuda.current_device())
-    if key not in _PAIR_ROOM:
-        L, room = _lib.lib_for(spec), ctypes.c_longlong(0)
-        _lib.check(L.gs_adjoint_paired_room(_METHOD_CODE[method], spec.code, K,
-                                            ctypes.addressof(room)), "gs_adjoint_paired_room", L)
-        _PAIR_ROOM[key] = room.value
-    return _PAIR_ROOM[key]
+    """Two warps per 32 trajectories: even batches whose blocks are all resident, short segments."""
+    return (not r.uneven and _pairs(r.spec.dim, r.n, None, None, "float64") and
+            all(rr.ckpt_every <= 2 for _rows, rr in _parts(r)))
 
 
 def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> bool:
@@ -1330,8 +1296,7 @@ def _few_steps(r) -> bool:
 
 def _lanes_for(r, saveat: bool) -> int:
     """Lanes per trajectory of r's split reverse pass, 0: not split."""
-    planned = all(rows is not None for rows, _rr in _parts(r))
-    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, saveat, r.method, planned)
+    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, saveat, r.method)
     return lanes if lanes and (r.method == METHOD_ROS23 or _few_steps(r)) else 0
 
 
@@ -1564,35 +1529,26 @@ def _replay_saveat_one(r: Record, y0: torch.Tensor, p: torch.Tensor, ts: torch.T
 
 def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
                    ybar: Optional[torch.Tensor] = None, *, want_y0: bool = True,
-def _split_work(r, words: int, device) -> Optional[dict]:
-    """The re-steps' workspaces of the split reverse pass, ``words`` doubles per trajectory, by the
-    part's id; None where there are none, or they do not fit (the unsplit passes need none).  They
-    come from the caller's stream's pool (a side stream's would be empty on its first use):
-    _over_parts orders the side streams after it and it after them, and they outlive the call."""
-    if not words or (8 * r.n * words > SPLIT_WORK_MAX and
-                     8 * r.n * words > _checkpoint_budget()):
-        return None
-    try:
-        return {id(rr): torch.empty(rr.n * words, dtype=torch.float64, device=device)
-                for _rows, rr in _parts(r)}
-    except torch.OutOfMemoryError:
-        return None
-
-
                    want_p: bool = True, precision: str = "float64", schedule: str = "auto"):
     """(dL/dy0, dL/dp) for cotangents ysbar = dL/dys (n, K, D) and ybar = dL/dy_final.
     ``schedule="auto"``, float64, where split_lanes says so: the split reverse pass; else it refills
     lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
     per trajectory for an even one."""
     lanes = _lanes_for(r, True) if r.n and _split_applies(r, precision, schedule) else 0
-    work = _split_work(r, ts.shape[-1] * (r.spec.dim + p.shape[1]), p.device) if lanes else None
-    if work is not None:
-        f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
-        res = _over_parts(r, lambda rr, rows: _adjoint_split(
-            rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
-            f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
-            work[id(rr)]))
-        return _scatter(r, res, 0), _scatter(r, res, 1)
+    if lanes:
+        words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
+        if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
+            f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
+            # the workspaces come from the caller's stream's pool (a side stream's would be empty
+            # on its first use): _over_parts orders the side streams after it and it after them,
+            # and `work` outlives the call
+            work = {id(rr): torch.empty(words // r.n * rr.n, dtype=torch.float64, device=p.device)
+                    for _rows, rr in _parts(r)}
+            res = _over_parts(r, lambda rr, rows: _adjoint_split(
+                rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
+                f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
+                work[id(rr)]))
+            return _scatter(r, res, 0), _scatter(r, res, 1)
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
     res = _over_parts(r, lambda rr, rows: _adjoint_saveat_one(
