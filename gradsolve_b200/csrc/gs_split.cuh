@@ -21,8 +21,7 @@
 // other trajectories share the batch; against one thread per trajectory they agree to rounding.
 //
 // B200, stiff Van der Pol batch (20,011 trajectories, 2269 steps on average, 17,220 the longest,
-// 64 saved times): reverse pass 9.9 ms with one lane each, 1.0 ms with 16; the whole closure
-// (with a record that holds every step at once) 48.9 -> 11.2 ms.
+// 64 saved times): reverse pass 8.8 ms with one lane each, 1.6 ms with 16.
 #pragma once
 #include <math_constants.h>
 
@@ -37,6 +36,7 @@ constexpr int kPoints = 4;  // consecutive requested times per thread of the sav
 // The forward quantities of one step, shared by the columns' VJPs.
 struct Tsit5Split {
   using Step = Tsit5F64Step;
+  static constexpr bool kRefine = false;
   template <class F>
   struct Fwd {
     StageStates<F> S;
@@ -55,6 +55,7 @@ struct Tsit5Split {
 
 struct Ros23Split {
   using Step = Ros23Step;
+  static constexpr bool kRefine = true;
   template <class F>
   struct Fwd {
     RosCore<F> c;
@@ -212,42 +213,19 @@ __device__ __forceinline__ bool takes_step(double dt) {
 }
 
 // ---- the split reverse pass ------------------------------------------------------------------
-// G lanes (a power of two, at most 32) per trajectory; order: as AdjointArgs.  kSave: with the
-// cotangents of dense output (a.ts, a.ysbar, work of saveat_vjp_kernel).
-template <class F, class S, bool kSave>
-__global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, int G,
-                                                            const double* work,
-                                                            const long long* order) {
-  constexpr int D = F::D, P = F::P, C = D + (kSave ? 1 : 0);
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int l = (int)(threadIdx.x & (unsigned)(G - 1));
-  long long j = tid / G;
-  const bool live = j < a.n;
-  if (!live) j = a.n - 1;  // (the lanes past the batch keep the warp's shuffles whole)
-  if (order) {
-    const long long o = __ldg(order + j);
-    j = (o >= 0 && o < a.n) ? o : -1;
-  }
-  const bool idle = j < 0;  // an entry of order outside the batch
-  if (idle) j = 0;
-  double p[P];
-#pragma unroll
-  for (int i = 0; i < P; ++i) p[i] = a.p[j * P + i];
-  const int na = live && !idle ? steps_in_record(a.n_acc, j, a.cap) : 0;
-  const int lo = (int)((long long)na * l / G), hi = (int)((long long)na * (l + 1) / G);
+// One sweep of a lane's steps [lo, hi) of trajectory j, latest first: their VJPs applied to the C
+// columns lam, gp; column C - 1 collects the re-steps' cotangents (kSave).  kfin: the number of
+// requested times of this lane's part and the ones before it.
+template <class F, class S, bool kSave, int C>
+__device__ __forceinline__ void split_sweep(const SaveatArgs& a, const double* work, long long j,
+                                            int na, int lo, int hi, const double* p,
+                                            double (&lam)[C][F::D], double (&gp)[C][F::P],
+                                            int& kfin) {
+  constexpr int D = F::D, P = F::P;
   const int K = a.ck_every;
-  double lam[C][D], gp[C][P];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-#pragma unroll
-    for (int i = 0; i < D; ++i) lam[c][i] = c == i ? 1.0 : 0.0;
-#pragma unroll
-    for (int i = 0; i < P; ++i) gp[c][i] = 0.0;
-  }
   // dense output: times [0, kk) not yet assigned; tlast = ts[kk - 1] (-inf without one)
   const double* ts = kSave ? a.ts + j * a.ts_ld : nullptr;
-  const double* ysb = kSave ? a.ysbar + j * (long long)a.K * D : nullptr;
-  int kk = 0, kfin = 0;  // kfin (the last lane's): the times at or past the end, from there on
+  int kk = 0;
   double tlast = -CUDART_INF;
   AdjBuf<D, D + 1> buf(K);
   int b = 0;
@@ -305,9 +283,9 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
           while (tlast > ts0) {
             const double* row = work + (j * (long long)a.K + (kk - 1)) * (D + P);
 #pragma unroll
-            for (int i = 0; i < D; ++i) lam[D][i] += row[i];
+            for (int i = 0; i < D; ++i) lam[C - 1][i] += row[i];
 #pragma unroll
-            for (int i = 0; i < P; ++i) gp[D][i] += row[D + i];
+            for (int i = 0; i < P; ++i) gp[C - 1][i] += row[D + i];
             --kk;
             tlast = kk > 0 ? ts[kk - 1] : -CUDART_INF;
           }
@@ -316,6 +294,56 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
     }
     b ^= 1;
   }
+}
+
+// G lanes (a power of two, at most 32) per trajectory; order: as AdjointArgs.  kSave: with the
+// cotangents of dense output (a.ts, a.ysbar, work of saveat_vjp_kernel).
+//
+// S::kRefine: a second sweep with the cotangents that the composition found.  Over a part of a
+// contracting (stiff) trajectory the columns are nearly parallel and the true cotangent may be
+// nearly orthogonal to what they have in common, so their sum cancels: on stiff Van der Pol
+// trajectories (17,000 steps, 8 lanes) rows were off by 5e-13 at the median and 2.6e-11 at most
+// against 80-bit arithmetic, where one thread per trajectory is off by 5e-14 and 1.5e-12.  The
+// second sweep runs each part from the cotangent at its end as one thread would; what it
+// leaves at the part before differs from that part's cotangent by the cancelled digits, and the
+// columns carry these differences through the parts: one thread's errors, for 1.6 to 1.9 times
+// the pass (20,011 trajectories of 2269 steps on average, 16 lanes, K = 8: 1.05 / 1.73 ms, with 64
+// saved times 1.32 / 2.25; one thread each, lanes refilled, 7.3 and 8.9).  Tsit5's trajectories
+// are not stiff for it (its errors against 80-bit arithmetic are one thread's on Van der Pol and on
+// Lorenz up to t = 70), and take one sweep.
+template <class F, class S, bool kSave>
+__global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, int G,
+                                                            const double* work,
+                                                            const long long* order) {
+  constexpr int D = F::D, P = F::P, C = D + (kSave ? 1 : 0);
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int l = (int)(threadIdx.x & (unsigned)(G - 1));
+  long long j = tid / G;
+  const bool live = j < a.n;
+  if (!live) j = a.n - 1;  // (the lanes past the batch keep the warp's shuffles whole)
+  if (order) {
+    const long long o = __ldg(order + j);
+    j = (o >= 0 && o < a.n) ? o : -1;
+  }
+  const bool idle = j < 0;  // an entry of order outside the batch
+  if (idle) j = 0;
+  double p[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) p[i] = a.p[j * P + i];
+  const int na = live && !idle ? steps_in_record(a.n_acc, j, a.cap) : 0;
+  const int lo = (int)((long long)na * l / G), hi = (int)((long long)na * (l + 1) / G);
+  double lam[C][D], gp[C][P];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) lam[c][i] = c == i ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < P; ++i) gp[c][i] = 0.0;
+  }
+  const double* ts = kSave ? a.ts + j * a.ts_ld : nullptr;
+  const double* ysb = kSave ? a.ysbar + j * (long long)a.K * D : nullptr;
+  int kfin = 0;  // (the last lane's: the times at or past the end, from there on)
+  split_sweep<F, S, kSave>(a, work, j, na, lo, hi, p, lam, gp, kfin);
   // the cotangent at the trajectory's end, from its last lane, through the parts in sequence
   double cur[D], in[D];
 #pragma unroll
@@ -330,7 +358,6 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
     }
   }
   const int base = (int)(threadIdx.x & 31u) & ~(G - 1);
-  if constexpr (kSave) kfin = __shfl_sync(0xffffffffu, kfin, base + G - 1);
 #pragma unroll
   for (int i = 0; i < D; ++i) cur[i] = __shfl_sync(0xffffffffu, cur[i], base + G - 1);
 #pragma unroll
@@ -352,12 +379,61 @@ __global__ void __launch_bounds__(128) adjoint_split_kernel(const SaveatArgs a, 
 #pragma unroll
     for (int i = 0; i < D; ++i) cur[i] = __shfl_sync(0xffffffffu, out[i], base + m);
   }
+  double own[P];  // the part's share of the parameter gradient
+  if constexpr (S::kRefine && D > 1) {  // (one component: nothing cancels)
+    double v[1][D], g[1][P], e[D], in_e[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) v[0][i] = in[i];
+#pragma unroll
+    for (int i = 0; i < P; ++i) g[0][i] = 0.0;
+    split_sweep<F, S, kSave>(a, work, j, na, lo, hi, p, v, g, kfin);
+    // e: what the cotangent at a part's end lacks; the last part's is exact
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      const double after = __shfl_down_sync(0xffffffffu, v[0][i], 1);
+      in_e[i] = l == G - 1 || after == in[i] ? 0.0 : after - in[i];
+      e[i] = 0.0;
+    }
+    for (int m = G - 1; m >= 0; --m) {
+#pragma unroll
+      for (int i = 0; i < D; ++i) e[i] += __shfl_sync(0xffffffffu, in_e[i], base + m);
+      if (l == m) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) in_e[i] = e[i];
+      }
+      double out[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        double x = lam[0][i] * e[0];
+#pragma unroll
+        for (int c = 1; c < D; ++c) x = x + lam[c][i] * e[c];
+        out[i] = x;
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) e[i] = __shfl_sync(0xffffffffu, out[i], base + m);
+    }
+#pragma unroll
+    for (int i = 0; i < D; ++i) cur[i] = v[0][i] + e[i];  // (of lane 0)
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      own[i] = g[0][i];
+#pragma unroll
+      for (int c = 0; c < D; ++c) own[i] = own[i] + gp[c][i] * in_e[c];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      double v = gp[0][i] * in[0];
+#pragma unroll
+      for (int c = 1; c < D; ++c) v = v + gp[c][i] * in[c];
+      if constexpr (kSave) v = v + gp[D][i];
+      own[i] = v;
+    }
+  }
+  if constexpr (kSave) kfin = __shfl_sync(0xffffffffu, kfin, base + G - 1);
 #pragma unroll
   for (int i = 0; i < P; ++i) {
-    double v = gp[0][i] * in[0];
-#pragma unroll
-    for (int c = 1; c < D; ++c) v = v + gp[c][i] * in[c];
-    if constexpr (kSave) v = v + gp[D][i];
+    double v = own[i];
     for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (a.gp && l == 0 && live && !idle) a.gp[j * P + i] = v;
   }

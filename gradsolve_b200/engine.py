@@ -1226,15 +1226,19 @@ _ADJ = {"auto": 0x000, "recompute": 0x400, "stages": 0x800, "pairs": 0xC00}
 # takes one, for a chain shorter by the number of lanes), or two warps per 32 trajectories
 # (csrc/gs_paired.cuh, up to 8 components: the one-thread arithmetic).  B200, reverse pass one
 # thread per trajectory / split / two warps:
-#   even batches: Lorenz (t = 1, 112 steps) n = 1024 68 / 25 us, 4096 68 / 39, 8192 48 / - / 29,
-#   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 442 / 45 us, 8192 449 / 197 / 326,
-#   16,384 452 / - / 385; HIRES 8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
-#   per-trajectory end times, 64 saved times: stiff Van der Pol 20,011 9.7 / 1.0 ms (16 lanes),
-#   200,000 11.8 / 9.9, 350,000 11.8 / 20.1; Van der Pol 100,000 1.37 / 0.67 ms (4), 200,000
-#   1.73 / 1.15, 350,000 1.66 / 2.01, 700,000 2.60 / 3.57 (one thread: lanes refilled);
-#   even batches, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
-#   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 392 / 230, 16,384
-#   409 / 667, 262,144 2.08 / 4.94 ms.
+#   one end time: Lorenz (t = 1, 112 steps) n = 1024 68 / 25 us, 4096 68 / 39, 8192 48 / - / 29,
+#   16,384 47 / 98 / 35, 32,768 49 / 90 / 53; Robertson 1024 185 / 43 / 134 us, 4096 191 / 99 / 138,
+#   8192 193 / 161 / 139; Van der Pol (Rosenbrock23, counts spread) 8192 606 / 191 / 524; HIRES
+#   8192 2323 / - / 1525 us, 16,384 2313 / - / 3019;
+#   per-trajectory end times (lanes refilled / split): Van der Pol 20,000 463 / 66 us, 65,536 701 /
+#   152, 131,072 784 / 279; with 64 saved times 100,000 1.37 / 0.67 ms (4 lanes), 200,000 1.73 / 1.15,
+#   350,000 1.66 / 2.01, 700,000 2.60 / 3.57;
+#   stiff Van der Pol (8 lanes, K = 2) in batch order 65,536 8.99 / 8.50 ms, 100,000 12.8 / 12.6, 131,072
+#   17.2 / 16.7; planned 131,072 8.7 / 6.6; with 64 saved times in batch order 65,536 11.3 / 9.4,
+#   100,000 14.6 / 14.8, 131,072 15.4 / 19.5; planned 100,000 11.2 / 7.3, 131,072 11.6 / 9.7;
+#   one end time, 64 saved times: Lorenz 4096 196 / 166 us, 16,384 199 / 378, 262,144 1.28 / 2.64
+#   ms; Lotka-Volterra 4096 169 / 137 us, 16,384 180 / 281; Robertson 4096 483 / 181, 8192 480 / 347;
+#   Van der Pol (Rosenbrock23) 4096 978 / 175.
 # The choice goes by the whole batch's size, so a tier of it takes the lanes of the others.  Tsit5
 # trajectories are split within SPLIT_TSIT5_STEPS steps taken: over thousands of steps of an
 # expanding flow (Lorenz, t = 70, gradients of 1e21) both evaluation orders are 1e-13 of a row
@@ -1248,16 +1252,21 @@ SPLIT_WORK_MAX = 1 << 30  # bytes of the re-steps' workspace taken without askin
 PAIRED = 0  # gs_adjoint_split's lanes argument for two warps
 
 
-def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5) -> int:
+def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD_TSIT5,
+                planned: bool = False) -> int:
     """Lanes per trajectory of the split reverse pass, 0: not split."""
+    ros = method == METHOD_ROS23
     if even:
         most = SPLIT_EVEN_SAVEAT_MAX if saveat else SPLIT_EVEN_MAX[method]
+    elif ros:
+        most = 1 << 17 if planned else 3 << 15
     else:
         most = 1 << (18 if saveat else 17)
     if dim > SPLIT_MAX_DIM or n > most:
         return 0
-    room = (1 << 16 if even and not saveat else 1 << 19) // max(n, 1)
-    return max(1, min(32, 1 << (room.bit_length() - 1) if room else 1))
+    room = ((1 << 17 if ros else 1 << 16) if even and not saveat else 1 << 19) // max(n, 1)
+    least = 8 if ros and not even else 1
+    return max(least, min(32, 1 << (room.bit_length() - 1) if room else 1))
 
 
 def _pairs(dim: int, n: int, t1v, saveat_ts, precision: str) -> bool:
@@ -1296,7 +1305,8 @@ def _few_steps(r) -> bool:
 
 def _lanes_for(r, saveat: bool) -> int:
     """Lanes per trajectory of r's split reverse pass, 0: not split."""
-    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, saveat, r.method)
+    planned = all(rows is not None for rows, _rr in _parts(r))
+    lanes = split_lanes(r.n, r.spec.dim, not r.uneven, saveat, r.method, planned)
     return lanes if lanes and (r.method == METHOD_ROS23 or _few_steps(r)) else 0
 
 

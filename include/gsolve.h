@@ -358,8 +358,13 @@ int gs_adjoint_saveat(int method, int field, int precision, long long n, const d
  * trajectory, or whose longest trajectories set the time.  Each lane runs its part's step VJPs
  * for the D unit cotangents and the parts are composed, D (+ 1) VJPs per step for a chain
  * `lanes` times shorter.  Float64, states of up to 3 components (GS_ERR_FIELD above).  work: n *
- * K * (D + P) doubles of scratch.  order: as gs_adjoint_ordered, or NULL.  Gradients agree with
- * the unsplit passes to rounding and depend on neither ckpt_every nor the rest of the batch.
+ * K * (D + P) doubles of scratch.  order: as gs_adjoint_ordered, or NULL.  Gradients depend on
+ * neither ckpt_every nor the rest of the batch.  They are another evaluation order of the unsplit
+ * passes' sums and no further than those from 80-bit arithmetic on the same states (Lorenz up to
+ * t = 70, Van der Pol, stiff Van der Pol over 17,000 steps, Robertson: 1e-13 of a row, 5e-12 at
+ * most, either way); the two differ by as much, and in components that are small beside their row
+ * by more of themselves.  Steps are those of the replay (K = 0: all that are not 0) or of dense
+ * output (those above 0).
  * lanes = 0 (K = 0, states of up to 8 components, segments that fit shared memory): two warps per
  * 32 trajectories instead, one recomputing the steps' forward quantities a segment ahead of the
  * other's VJPs -- the unsplit pass's arithmetic.  No counterpart in the reference.
