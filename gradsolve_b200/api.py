@@ -256,9 +256,12 @@ def _solve_saveat(name, problem, y0, params, saveat, *, rtol, atol, device, max_
     t1s, t1v = _t1_arg(problem, t1, dev)
     ts = validate_saveat(saveat, float(problem.t0), t1s, _t1_host(problem, t1)[1], y0_t.shape[0])
     ms = int(max_steps or DEFAULT_MAX_STEPS[name])
-    # the forward re-steps each saved time as it integrates: no replay pass
+    # the forward gives the saved states: no replay pass, and no use for the checkpoints but theirs
+    # (the longest interval that those states are quick from, unless memory is short)
+    K = engine.choose_ckpt_every("auto", spec.dim, y0_t.shape[0], min(engine.DEFAULT_CAP0, ms), None,
+                                 engine.SAVEAT_CKPT_MAX)
     r = engine.forward_record(method, spec, y0_t, pk, t0=float(problem.t0), t1=t1s, t1v=t1v,
-                              rtol=rtol, atol=atol, max_steps=ms, checkpoint="sqrt",
+                              rtol=rtol, atol=atol, max_steps=ms, checkpoint=K,
                               saveat_ts=torch.as_tensor(ts, device=dev))
     engine.raise_on_failed(r, ms, t1s)
     yf, ys = r.y_final, r.ys

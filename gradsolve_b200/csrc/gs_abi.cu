@@ -1769,7 +1769,39 @@ int launch_saveat_states(const gs::RecordArgs& a, cudaStream_t s) {
   gs::saveat_states_kernel<F, M><<<grid_for(a.n * parts), kBlock, 0, s>>>(b);
   return cuda_check("saveat_states_kernel");
 }
-bool states_apart(const gs::RecordArgs& a) { return a.ys && a.rec && a.ckpt; }
+// The pass of its own walks K / 2 steps from a checkpoint to a requested time where the forward
+// has the state at hand, so it loses where those steps cost more than the lanes that wait: long
+// intervals, and batches that fill the chip.  B200, forward with its 64 times, in the forward /
+// apart, us, at K = 2, 8, 32:
+//   one end time: Lorenz 4096 171 / 144, 169 / 149, 167 / 161   8192 175 / 152, 170 / 157, 171 / 185
+//               16,384 177 / 173, 177 / 188, 180 / 237   262,144 906 / 999, 782 / 1242, 762 / 1992
+//   Lotka-Volterra 16,384 178 / 146, 177 / 159, 171 / 197   65,536 254 / 273, 262 / 297, 255 / 451
+//   Lorenz-96 of 8 2048 228 / 159, 229 / 167, 224 / 187   8192 231 / 195, 230 / 220, 231 / 281
+//               16,384 250 / 258, 250 / 287, 245 / 425
+//   Robertson 16,384 448 / 337, 438 / 334, 432 / 423   262,144 2321 / 2118, 2277 / 2238, 2248 / 3431
+//   HIRES 1024 701 / 652, 688 / 650, 692 / 693   4096 714 / 693, 702 / 701, 701 / 801
+//               8192 715 / 768, 705 / 777, 702 / 955
+//   per-trajectory end times (lanes refilled, each re-step at its own attempt): Van der Pol 100,000
+//               1449 / 1126, 1435 / 1129, 1372 / 1277   524,288 3383 / 2706, 3353 / 2746, 3321 / 3494
+//   Lorenz 32,768 334 / 220, 316 / 240, 317 / 335   262,144 1107 / 993, 1096 / 1179, 1095 / 1894
+//   Lorenz-96 of 8 8192 333 / 184, 331 / 200, 334 / 266   32,768 457 / 370, 458 / 417, 455 / 633
+//               262,144 2673 / 1944, 2660 / 2323, 2657 / 3863
+//   Robertson 32,768 648 / 426, 641 / 436, 633 / 595   131,072 1399 / 1237, 1360 / 1294, 1341 / 1882
+//   HIRES 8192 1113 / 802, 1087 / 804, 1071 / 1009   32,768 1363 / 1348, 1331 / 1464, 1316 / 2196
+template <class F>
+bool states_apart(const gs::RecordArgs& a, bool stiff) {
+  if (!a.ys || !a.rec || !a.ckpt) return false;
+  constexpr bool small = F::D <= 3;
+  const bool close = a.ck_every <= 8;
+  const long long n = a.n, nk = a.n * a.ck_every;
+  if (a.t1v) {
+    if (small) return close || nk <= (1 << 20);
+    return stiff ? n <= (1 << 13) || nk <= (1 << 16) : close || nk <= (1 << 18);
+  }
+  if (small && stiff) return close || nk <= (1 << 19);
+  if (small) return n <= (1 << 14) && nk <= (1 << 16);
+  return stiff ? n <= (1 << 12) && nk <= (1 << 15) : n <= (1 << 13) && nk <= (1 << 16);
+}
 
 template <class F>
 int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed, FwdLanes lanes,
@@ -1778,7 +1810,8 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
     return coop_refuse<F>("the dense output (saveat)");
   } else {
     if (mixed) return launch_fwd_lanes<F, gs::LaneTsit5Mixed<F>>(a, s, lanes);
-    if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
+    if (!states_apart<F>(a, false))
+      return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
     gs::RecordArgs b = a;
     b.ys = nullptr;
     const int sched = lanes == kStatic ? GS_SCHED_STATIC
@@ -1791,7 +1824,7 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
 template <class F>
 int launch_fwd_saveat_ros23(const gs::RecordArgs& a, cudaStream_t s, FwdLanes lanes,
                             int precision) {
-  if (!states_apart(a)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
+  if (!states_apart<F>(a, true)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
   gs::RecordArgs b = a;
   b.ys = nullptr;
   const int sched = lanes == kStatic ? GS_SCHED_STATIC
