@@ -79,6 +79,7 @@ _SIGS = {
     "gs_adjoint_split": (c_int, [c_int, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_int,
                                  c_void_p, c_int, c_int, c_void_p, c_ll, c_int, c_void_p,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "gs_adjoint_paired_room": (c_int, [c_int, c_int, c_int, c_void_p]),
     "gs_tsit5_vjp_static": (c_int, [c_int, c_ll, c_void_p, c_void_p, c_double, c_void_p, c_ll,
                                     c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
 }

@@ -1876,6 +1876,43 @@ int launch_adjoint_paired(const gs::SaveatArgs& a, cudaStream_t s, const long lo
   return cuda_check("adjoint_paired_kernel");
 }
 
+// Trajectories that are resident at once with two warps per 32 of them; 0 where that pass is not
+// built or does not fit.  A dense W of more than 3 components (pivoted LU) takes it at K = 2
+// alone: at K = 1 one thread per trajectory is faster at every size (8 components 1756 / 2348 us
+// at 2048), and 128,000 bytes a block leave one per SM (K = 2: 4096 2362 / 2180 us, 4736 2524 /
+// 2604, 8192 2369 / 4450).
+template <class F, class S>
+int paired_room(int K, bool dense_w, long long* room) {
+  const int sd = gs::paired_smem_doubles<F, S>(K);
+  const size_t smem = (size_t)sd * 64 * sizeof(double);
+  *room = 0;
+  if (smem > kSegBudget || (dense_w && K == 1)) return GS_OK;
+  int rc, dev = 0, sms = 0, per_sm = 0;
+  if ((rc = allow_smem(gs::adjoint_paired_kernel<F, S>, smem))) return rc;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs::adjoint_paired_kernel<F, S>, 64,
+                                                      smem);
+  if (e != cudaSuccess)
+    return fail(GS_ERR_CUDA, std::string("CUDA: occupancy query: ") + cudaGetErrorString(e));
+  *room = 32ll * per_sm * sms;
+  return GS_OK;
+}
+template <class F>
+int paired_room_tsit5(int K, long long* room) {
+  if constexpr (F::D <= 8) return paired_room<F, gs::Tsit5Pair<F>>(K, false, room);
+  *room = 0;
+  return GS_OK;
+}
+template <class F>
+int paired_room_ros23(int K, long long* room) {
+  if constexpr (F::D <= 8)
+    return paired_room<F, gs::Ros23Pair<F>>(K, gs::Ros23Pair<F>::kPiv > 0, room);
+  *room = 0;
+  return GS_OK;
+}
+
 template <class F>
 int launch_split_tsit5(const gs::SaveatArgs& a, cudaStream_t s, int lanes, double* work,
                        const long long* order) {
@@ -2024,6 +2061,20 @@ extern "C" int gs_adjoint_split(int method, int field, int precision, long long 
   }
   if (method == GS_METHOD_ROS23) {
     GS_ROS23_DISPATCH(field, launch_split_ros23, a, s, lanes, work, order)
+  }
+  return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
+}
+
+extern "C" int gs_adjoint_paired_room(int method, int field, int ckpt_every, long long* room) {
+  const char* who = "gs_adjoint_paired_room";
+  if (!room || ckpt_every < 1 || ckpt_every > gs::KMAX)
+    return fail(GS_ERR_ARG, std::string(who) + ": room and an interval in [1, " +
+                                std::to_string(gs::KMAX) + "] are required");
+  if (method == GS_METHOD_TSIT5) {
+    GS_TSIT5_DISPATCH(field, paired_room_tsit5, ckpt_every, room)
+  }
+  if (method == GS_METHOD_ROS23) {
+    GS_ROS23_DISPATCH(field, paired_room_ros23, ckpt_every, room)
   }
   return fail(GS_ERR_ARG, std::string(who) + ": unknown method " + std::to_string(method));
 }

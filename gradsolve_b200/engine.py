@@ -245,13 +245,20 @@ def tuned_ckpt_every(method: str, spec: FieldSpec, precision: str) -> Optional[i
     return _TUNED.get((method, spec.key, precision))
 
 
+def _own_interval(method: str, spec: FieldSpec, n: int, precision: str, t1v, saveat_ts) -> bool:
+    """Batches whose reverse pass runs two warps per 32 trajectories take the interval it is built
+    for, 2, and not the one tuned on larger ones."""
+    return (precision == "float64" and t1v is None and saveat_ts is None and
+            _pairs(method, spec, n))
+
+
 def auto_ckpt_every(method: str, spec: FieldSpec, n: int, precision: str, t1v,
                     saveat_ts) -> Optional[int]:
     """The interval checkpoint="auto" starts from (choose_ckpt_every's ``tuned``)."""
     tuned = tuned_ckpt_every(method, spec, precision)
     if precision != "float64":
         return tuned
-    if tuned is None or _pairs(spec.dim, n, t1v, saveat_ts, precision):
+    if tuned is None or _own_interval(method, spec, n, precision, t1v, saveat_ts):
         tuned = 2  # (a small batch: its checkpoints are no matter)
     # (dense output walks K / 2 steps from a checkpoint per requested time)
     return tuned if saveat_ts is None else min(tuned, SAVEAT_CKPT_MAX)
@@ -932,7 +939,7 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
         autotune_lanes(spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                        max_steps=max_steps)
     if (checkpoint == "auto" and tuned_ckpt_every(method, spec, precision) is None and
-            n >= 4096 and not _pairs(spec.dim, n, t1v, saveat_ts, precision)):
+            n >= 4096 and not _own_interval(method, spec, n, precision, t1v, saveat_ts)):
         autotune_ckpt_every(method, spec, y0, p, t0=t0, t1=t1, t1v=t1v, rtol=rtol, atol=atol,
                             max_steps=max_steps, precision=precision)
     occ_sched = "static" if method == METHOD_ROS23 and schedule == "auto" and isinstance(
@@ -1269,17 +1276,34 @@ def split_lanes(n: int, dim: int, even: bool, saveat: bool, method: str = METHOD
     return max(least, min(32, 1 << (room.bit_length() - 1) if room else 1))
 
 
-def _pairs(dim: int, n: int, t1v, saveat_ts, precision: str) -> bool:
-    """Batches of the sizes that two warps per 32 trajectories are for: they take the interval that
-    pass is built for, K = 2, and not the one tuned on larger ones."""
-    most = 1 << 14 if dim <= 4 else 1 << 13 if dim <= 8 else 0
-    return 0 < n <= most and t1v is None and saveat_ts is None and precision == "float64"
+def _pairs(method: str, spec: FieldSpec, n: int, K: int = 2) -> bool:
+    """Whether an even batch is of a size that two warps per 32 trajectories are for: up to 2^14 (2^13
+    above 4 components) and 7/8 of what is resident at once, short of a second wave (Rosenbrock23
+    with a dense W of 8 components, one block per SM: 4096 2362 / 2180 us, 4736, the whole wave,
+    2524 / 2604, 5000 2446 / 3462)."""
+    most = 1 << 14 if spec.dim <= 4 else 1 << 13 if spec.dim <= 8 else 0
+    return 0 < n <= most and K <= 2 and 8 * n <= 7 * _pair_room(method, spec, K)
 
 
 def _paired(r) -> bool:
-    """Two warps per 32 trajectories: even batches whose blocks are all resident, short segments."""
-    return (not r.uneven and _pairs(r.spec.dim, r.n, None, None, "float64") and
-            all(rr.ckpt_every <= 2 for _rows, rr in _parts(r)))
+    """r's reverse pass runs two warps per 32 trajectories."""
+    return not r.uneven and all(_pairs(r.method, r.spec, r.n, rr.ckpt_every)
+                                for _rows, rr in _parts(r))
+
+
+_PAIR_ROOM: dict = {}  # (method, field key, interval, device) -> gs_adjoint_paired_room
+
+
+def _pair_room(method: str, spec: FieldSpec, K: int) -> int:
+    if not torch.cuda.is_initialized():
+        return 0
+    key = (method, spec.key, K, torch.cuda.current_device())
+    if key not in _PAIR_ROOM:
+        L, room = _lib.lib_for(spec), ctypes.c_longlong(0)
+        _lib.check(L.gs_adjoint_paired_room(_METHOD_CODE[method], spec.code, K,
+                                            ctypes.addressof(room)), "gs_adjoint_paired_room", L)
+        _PAIR_ROOM[key] = room.value
+    return _PAIR_ROOM[key]
 
 
 def _split_applies(r, precision: str, schedule: str, variant: str = "auto") -> bool:

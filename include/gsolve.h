@@ -376,6 +376,13 @@ int gs_adjoint_split(int method, int field, int precision, long long n, const do
                      double* gp, const long long* order, void* stream);
 
 /*
+ * How many trajectories are resident on the current device at once with gs_adjoint_split's two
+ * warps (lanes = 0) at this interval: *room, 0 where that pass is not built, does not fit or is
+ * not the faster one at any size.  No counterpart in the reference.
+ */
+int gs_adjoint_paired_room(int method, int field, int ckpt_every, long long* room);
+
+/*
  * Record conversion between the reference's padded (n, S) layout (row j = trajectory j's
  * accepted dts, zero padded; gradsolve/warp/warp_replay.py:181-182) and the chunked record.
  * from_padded also writes n_steps[j] = index of the last non-zero dt + 1 (zero steps
