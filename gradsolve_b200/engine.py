@@ -971,9 +971,12 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
 
 # Fresh batches from these sizes up run the compacting forward (gs_fwd_record_compact,
 # csrc/gs_compact.cuh): their step counts are not known yet, and where they spread a third of the
-# one-launch forward's lanes idle.  Below, its launches' tails cost what it saves: Robertson 65,536
-# 1.06 / 1.00 ms, Lotka-Volterra (float32 stages) 65,536 137 / 164 us, 2^18 388 / 374 us.
-COMPACT_MIN = {METHOD_TSIT5: 1 << 18, METHOD_ROS23: 1 << 16}
+# one-launch forward's lanes idle.  Below, its launches' tails cost what it saves, us, one launch /
+# compacting: Rosenbrock23 Robertson 32,768 278 / 332, 65,536 463 / 477, 131,072 732 / 701, 2^18
+# 1388 / 1247; Van der Pol (stiff, a few long trajectories) 65,536 1097 / 1352, 131,072 2057 / 2172,
+# 2^18 3545 / 3575; Tsit5 Lotka-Volterra 131,072 256 / 262, 2^18 433 / 398; Van der Pol 131,072 303 /
+# 308, 2^18 551 / 500, 2^19 1049 / 865; Lorenz 2^18 1318 / 1294.
+COMPACT_MIN = {METHOD_TSIT5: 1 << 18, METHOD_ROS23: 1 << 17}
 COMPACT_MAX_DIM = 4
 
 
@@ -985,7 +988,7 @@ def _compacts(method, spec, n, precision, schedule, t1v, saveat_ts) -> bool:
 
 
 def _compact_work(L, code, n, device) -> Optional[torch.Tensor]:
-    """Scratch of the compacting forward, 30 to 80 bytes a trajectory; None where it does not
+    """Scratch of the compacting forward, 28 to 88 bytes a trajectory; None where it does not
     fit (the one-launch forward needs none)."""
     size = L.gs_fwd_compact_bytes(*code, n)
     try:
