@@ -1564,6 +1564,21 @@ def _replay_saveat_one(r: Record, y0: torch.Tensor, p: torch.Tensor, ts: torch.T
     return yf, ys
 
 
+def _split_work(r, words: int, device) -> Optional[dict]:
+    """The re-steps' workspaces of the split reverse pass, ``words`` doubles per trajectory, by the
+    part's id; None where there are none, or they do not fit (the unsplit passes need none).  They
+    come from the caller's stream's pool (a side stream's would be empty on its first use):
+    _over_parts orders the side streams after it and it after them, and they outlive the call."""
+    if not words or (8 * r.n * words > SPLIT_WORK_MAX and
+                     8 * r.n * words > _checkpoint_budget()):
+        return None
+    try:
+        return {id(rr): torch.empty(rr.n * words, dtype=torch.float64, device=device)
+                for _rows, rr in _parts(r)}
+    except torch.OutOfMemoryError:
+        return None
+
+
 def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
                    ybar: Optional[torch.Tensor] = None, *, want_y0: bool = True,
                    want_p: bool = True, precision: str = "float64", schedule: str = "auto"):
@@ -1572,20 +1587,14 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
     lanes from a work counter for an uneven batch (per-trajectory end times) and runs one thread
     per trajectory for an even one."""
     lanes = _lanes_for(r, True) if r.n and _split_applies(r, precision, schedule) else 0
-    if lanes:
-        words = r.n * ts.shape[-1] * (r.spec.dim + p.shape[1])
-        if ts.shape[-1] and (8 * words <= SPLIT_WORK_MAX or 8 * words <= _checkpoint_budget()):
-            f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
-            # the workspaces come from the caller's stream's pool (a side stream's would be empty
-            # on its first use): _over_parts orders the side streams after it and it after them,
-            # and `work` outlives the call
-            work = {id(rr): torch.empty(words // r.n * rr.n, dtype=torch.float64, device=p.device)
-                    for _rows, rr in _parts(r)}
-            res = _over_parts(r, lambda rr, rows: _adjoint_split(
-                rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
-                f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
-                work[id(rr)]))
-            return _scatter(r, res, 0), _scatter(r, res, 1)
+    work = _split_work(r, ts.shape[-1] * (r.spec.dim + p.shape[1]), p.device) if lanes else None
+    if work is not None:
+        f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
+        res = _over_parts(r, lambda rr, rows: _adjoint_split(
+            rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
+            f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
+            work[id(rr)]))
+        return _scatter(r, res, 0), _scatter(r, res, 1)
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
     res = _over_parts(r, lambda rr, rows: _adjoint_saveat_one(
