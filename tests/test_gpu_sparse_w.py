@@ -142,3 +142,27 @@ def test_tiny_scales(gslib, cuda, method, field, schedule):
             r.n_rej.tolist() == [int(r.n_rej[0])] * 3
         scaled = r.y_final / y0
         assert float((scaled / scaled[0] - 1.0).abs().max()) <= 1e-9
+
+
+def test_two_warps_with_exchanged_pivots(gslib, cuda):
+    """The two-warp reverse pass over a sparse W whose pivots do not hold on some steps: those run
+    the pivoted elimination out of line in both warps."""
+    import gradsolve_b200 as gsb
+    from gradsolve_b200 import engine
+    D = 8
+    A = _matrix("pivots", D)
+    spec = gsb.register_linstiff(f"linstiff_sparse_pivots_{D}", A)
+    rng = np.random.default_rng(3)
+    n = 70
+    y0 = torch.tensor(rng.uniform(-1.0, 1.0, (n, D)), device=cuda)
+    p = torch.zeros((n, spec.nparam), dtype=torch.float64, device=cuda)
+    for K in (1, 2):
+        r = engine.forward_record("rosenbrock23", spec, y0, p, t0=0.0, t1=4.0, rtol=1e-3,
+                                  atol=1e-5, checkpoint=K)
+        assert _exchanges(A, r.padded_dts().cpu().numpy()) > 0
+        ybar = 2.0 * r.y_final
+        ref = engine.adjoint(r, p, ybar, schedule="static")[0]
+        got = engine._adjoint_split(r, engine.PAIRED, p, ybar, None, None, True, True, None)[0]
+        # two float64 evaluation orders of the same sums, as in test_gpu_split.py
+        rel = ((got - ref).abs().max(1).values / ref.abs().max(1).values).max()
+        assert float(rel) <= 1e-10, K
