@@ -245,20 +245,29 @@ def tuned_ckpt_every(method: str, spec: FieldSpec, precision: str) -> Optional[i
     return _TUNED.get((method, spec.key, precision))
 
 
-def _own_interval(method: str, spec: FieldSpec, n: int, precision: str, t1v, saveat_ts) -> bool:
-    """Batches whose reverse pass runs two warps per 32 trajectories take the interval it is built
-    for, 2, and not the one tuned on larger ones."""
-    return (precision == "float64" and t1v is None and saveat_ts is None and
-            _pairs(method, spec, n))
+def _own_interval(method: str, spec: FieldSpec, n: int, precision: str, t1v,
+                  saveat_ts) -> Optional[int]:
+    """The interval of batches whose reverse pass is not the one-thread one that the tuner times, or
+    None: 2, which two warps per 32 trajectories are built for, and for the split pass of uneven
+    batches what it was fastest at (K = 2, 4, 8, 16: Van der Pol 100,000 with 64 saved times 564,
+    566, 601, 756 us; stiff Van der Pol 20,011 2.96, -, 2.25, - ms, planned 2.50, 1.77, 1.65, 1.88)."""
+    if precision != "float64":
+        return None
+    if t1v is None:
+        return 2 if saveat_ts is None and _pairs(method, spec, n) else None
+    if split_lanes(n, spec.dim, False, saveat_ts is not None, method):
+        return 8 if method == METHOD_ROS23 else 4
+    return None
 
 
 def auto_ckpt_every(method: str, spec: FieldSpec, n: int, precision: str, t1v,
                     saveat_ts) -> Optional[int]:
     """The interval checkpoint="auto" starts from (choose_ckpt_every's ``tuned``)."""
-    tuned = tuned_ckpt_every(method, spec, precision)
+    own = _own_interval(method, spec, n, precision, t1v, saveat_ts)
+    tuned = own or tuned_ckpt_every(method, spec, precision)
     if precision != "float64":
         return tuned
-    if tuned is None or _own_interval(method, spec, n, precision, t1v, saveat_ts):
+    if tuned is None:
         tuned = 2  # (a small batch: its checkpoints are no matter)
     # (dense output walks K / 2 steps from a checkpoint per requested time)
     return tuned if saveat_ts is None else min(tuned, SAVEAT_CKPT_MAX)

@@ -66,3 +66,22 @@ def test_small_even_batches_have_their_own_interval(gslib, cuda, tables, method,
     assert engine.forward_record(method, spec, y0, p, **kw).ckpt_every == 2
     y0, p = _batch(cuda, field, (1 << 14) + 1)
     assert engine.forward_record(method, spec, y0, p, **kw).ckpt_every == 12
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("method,field,want", [("tsit5", "lorenz", 4),
+                                               ("rosenbrock23", "robertson", 8)])
+def test_uneven_split_batches_have_their_own_interval(gslib, cuda, tables, method, field, want,
+                                                      dense):
+    from gradsolve_b200 import engine
+    from gradsolve_b200.fields import field_spec
+    spec, n = field_spec(field), 5000
+    key = (method, spec.key, "float64")
+    y0, p = _batch(cuda, field, n)
+    t1v = torch.linspace(0.1, 1.0, n, device=cuda, dtype=torch.float64)
+    kw = dict(t0=0.0, t1=1.0, rtol=1e-6, atol=1e-9, t1v=t1v,
+              saveat_ts=t1v[:, None] * 0.5 if dense else None)
+    assert engine.forward_record(method, spec, y0, p, **kw).ckpt_every == want
+    assert key not in engine._TUNED
+    engine._TUNED[key] = 16
+    assert engine.forward_record(method, spec, y0, p, **kw).ckpt_every == want
