@@ -984,12 +984,13 @@ def forward_record(method: str, spec: FieldSpec, y0: torch.Tensor, p: torch.Tens
                          ws.n_rej, ws.status, uneven=ws.uneven, ys=ws.ys, streams=[None])
         return _forward_planned(method, spec, y0, p, t1v, saveat_ts, plan, kw)
     cap = max(1, min(int(cap0), int(max_steps)))
-    r0 = _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw,
-                      compact=_compacts(method, spec, n, precision, schedule, t1v, saveat_ts))
+    compact = (_compacts(method, spec, n, precision, schedule, t1v, saveat_ts) and
+               _compaction_pays(method, spec, y0, p, cap, kw))
+    r0 = _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=compact)
     return _grow(method, spec, y0, p, t1v, saveat_ts, r0, None, kw)
 
 
-# Fresh batches from these sizes up run the compacting forward (gs_fwd_record_compact,
+# Fresh batches from these sizes up may run the compacting forward (gs_fwd_record_compact,
 # csrc/gs_compact.cuh): their step counts are not known yet, and where they spread a third of the
 # one-launch forward's lanes idle.  Below, its launches' tails cost what it saves, us, one launch /
 # compacting: Rosenbrock23 Robertson 32,768 278 / 332, 65,536 463 / 477, 131,072 732 / 701, 2^18
@@ -1005,6 +1006,46 @@ def _compacts(method, spec, n, precision, schedule, t1v, saveat_ts) -> bool:
             t1v is None and saveat_ts is None and (method, spec.key) not in _OCC_PINNED and
             not _IN_TUNER[0] and
             (precision == "float64" or (precision == "mixed" and method == METHOD_TSIT5)))
+
+
+# From those sizes it depends on the field and on how its counts spread, and the share of idle lanes
+# alone does not tell (us, one launch of the tuned instance / compacting; share of idle lanes):
+# Lotka-Volterra 2^18 0 278 / 299, 0.15 323 / 346, 0.29 430 / 428, 2^20 0.29 1374 / 1253; Van der Pol
+# (mu = 2 to 6) 2^18 0.24 1206 / 1294, 2^20 3990 / 4427; Lorenz 2^18 0.33 2684 / 2948, 2^20 0.23 9633 /
+# 9104; Lorenz-96 of 4 2^18 0.15 1217 / 1238, 0.30 1583 / 1511; Robertson 2^18 0 2148 / 2180, 0.31
+# 3302 / 2855.  So both are timed, once per field, precision and power of two of the size, on the
+# first such batch, as the other choices are; one launch unless the other is faster by a margin.
+_COMPACT: dict = {}  # (method, field key, precision, n.bit_length()) -> bool
+COMPACT_SAMPLE = 1 << 20
+COMPACT_MARGIN = 0.01
+
+
+@_tuner
+def _time_compaction(method, spec, y0, p, cap, kw) -> bool:
+    # (a workspace's own buffers for both, and nothing read on the host between the events)
+    m = min(y0.shape[0], COMPACT_SAMPLE)
+    y0, p = y0[:m].contiguous(), p[:m].contiguous()
+    box = [None]
+
+    def once(compact):
+        box[0] = _forward_one(method, spec, y0, p, None, None, cap, box[0], kw, compact=compact)
+
+    ms = {}
+    for reps in (1, 2, 2):  # in turn; the first is to warm up
+        for compact in (False, True):
+            t = _time_ms(lambda: once(compact), reps)
+            ms[compact] = t if reps == 1 else min(ms[compact], t)
+    return ms[True] < ms[False] * (1.0 - COMPACT_MARGIN)
+
+
+def _compaction_pays(method, spec, y0, p, cap, kw) -> bool:
+    key = (method, spec.key, kw["precision"], y0.shape[0].bit_length())
+    if key not in _COMPACT:
+        try:
+            _COMPACT[key] = _time_compaction(method, spec, y0, p, cap, kw)
+        except torch.OutOfMemoryError:
+            return False
+    return _COMPACT[key]
 
 
 def _compact_work(L, code, n, device) -> Optional[torch.Tensor]:
