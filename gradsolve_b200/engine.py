@@ -568,6 +568,28 @@ def _status_max(status: torch.Tensor, device) -> int:
     return int(vals[0])
 
 
+# Small batches whose reverse pass asks for the longest step count (_few_steps) have it read in the
+# same copy: a read of its own is another synchronisation (a closure of 1024 Lorenz trajectories
+# 382 us without the question, 399 with it asked apart).  Above, the one reduction over both costs
+# more than it saves (2^20: 390 us).
+COUNTS_READ_MAX = 1 << 14
+
+
+def _read_status(r) -> int:
+    """_status_max of a Record, and its steps_max where its reverse pass will ask for it."""
+    n_most = COUNTS_READ_MAX if r.uneven else SPLIT_EVEN_SAVEAT_MAX
+    if (r.method == METHOD_ROS23 or r.cap <= SPLIT_TSIT5_STEPS or r.spec.dim > SPLIT_MAX_DIM or
+            r.n > n_most or r.rec.element_size() != 8 or r.steps_max is not None):
+        return _status_max(r.status, r.status.device)
+    both = torch.stack((r.status, r.n_acc)).amax(1)
+    c = _BAD_MOVES.get(r.status.device.index)
+    vals = (both if c is None else torch.cat([both.to(torch.int64), c])).tolist()
+    if c is not None and vals[2] != 0:
+        _raise_bad_moves(c, int(vals[2]))
+    r.steps_max = int(vals[1])
+    return int(vals[0])
+
+
 def _movable(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dtype in _ELEM_BYTES and t.is_contiguous() and t.ndim >= 1
 
@@ -1144,7 +1166,7 @@ def _grow(method, spec, y0, p, t1v, saveat_ts, r0, streams, kw):
     max_steps = int(kw["max_steps"])
     if n == 0 or r0.cap >= max_steps:
         return r0
-    r0.status_max = _status_max(r0.status, y0.device)
+    r0.status_max = _read_status(r0)
     if r0.status_max < 3:  # no row overflowed the record
         return r0
     rows = torch.nonzero(r0.status == 3).squeeze(1)
@@ -1232,7 +1254,8 @@ def raise_on_failed(r: Record, max_steps: int, t1) -> None:
     if r.n == 0:
         return
     if r.status_max is None:  # (a record of max_steps capacity: the forward read no status)
-        r.status_max = _status_max(r.status, r.status.device)
+        r.status_max = (_read_status(r) if isinstance(r, Record) else
+                        _status_max(r.status, r.status.device))
     if r.status_max == 0:
         return
     bad = torch.nonzero(r.status != 0).flatten()
