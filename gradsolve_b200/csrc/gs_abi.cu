@@ -1788,9 +1788,11 @@ int launch_saveat_states(const gs::RecordArgs& a, cudaStream_t s) {
 //               262,144 2673 / 1944, 2660 / 2323, 2657 / 3863
 //   Robertson 32,768 648 / 426, 641 / 436, 633 / 595   131,072 1399 / 1237, 1360 / 1294, 1341 / 1882
 //   HIRES 8192 1113 / 802, 1087 / 804, 1071 / 1009   32,768 1363 / 1348, 1331 / 1464, 1316 / 2196
+// (A batch ordered by cost has other lines; its caller names the route.)
 template <class F>
-bool states_apart(const gs::RecordArgs& a, bool stiff) {
+bool states_apart(const gs::RecordArgs& a, bool stiff, int precision) {
   if (!a.ys || !a.rec || !a.ckpt) return false;
+  if (precision & GS_SAVEAT_MASK) return (precision & GS_SAVEAT_MASK) == GS_SAVEAT_APART;
   constexpr bool small = F::D <= 3;
   const bool close = a.ck_every <= 8;
   const long long n = a.n, nk = a.n * a.ck_every;
@@ -1810,7 +1812,7 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
     return coop_refuse<F>("the dense output (saveat)");
   } else {
     if (mixed) return launch_fwd_lanes<F, gs::LaneTsit5Mixed<F>>(a, s, lanes);
-    if (!states_apart<F>(a, false))
+    if (!states_apart<F>(a, false, precision))
       return launch_fwd_lanes<F, gs::LaneTsit5F64<F>>(a, s, lanes);
     gs::RecordArgs b = a;
     b.ys = nullptr;
@@ -1824,7 +1826,8 @@ int launch_fwd_saveat_tsit5(const gs::RecordArgs& a, cudaStream_t s, bool mixed,
 template <class F>
 int launch_fwd_saveat_ros23(const gs::RecordArgs& a, cudaStream_t s, FwdLanes lanes,
                             int precision) {
-  if (!states_apart<F>(a, true)) return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
+  if (!states_apart<F>(a, true, precision))
+    return launch_fwd_lanes<F, gs::LaneRos23<F>>(a, s, lanes);
   gs::RecordArgs b = a;
   b.ys = nullptr;
   const int sched = lanes == kStatic ? GS_SCHED_STATIC

@@ -33,6 +33,9 @@ _PREC = {"float64": _lib.GS_PREC_F64, "mixed": _lib.GS_PREC_MIXED,
 # scheduling flags (include/gsolve.h GS_SCHED_*): one thread per trajectory, persistent lanes
 # refilled from a work counter, or persistent lanes with strided assignment
 _SCHED = {"auto": 0x000, "static": 0x100, "refill": 0x200, "strided": 0x300}
+# how a float64 forward takes its dense output (GS_SAVEAT_*): by the library's rule on sizes, as it
+# integrates, or by a kernel of its own from the checkpoints
+_DENSE = {"auto": 0x000000, "within": 0x080000, "apart": 0x100000}
 
 # default record capacity before growth (the reference's device recorder starts at 1024)
 DEFAULT_CAP0 = 1024
@@ -1080,9 +1083,11 @@ def _compact_work(L, code, n, device) -> Optional[torch.Tensor]:
         return None
 
 
-def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False) -> Record:
+def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False,
+                 dense="auto") -> Record:
     """One record of capacity ``cap`` for all rows of y0 (buffers reused from ws if they
-    match), on the current stream; ``compact``: by the compacting forward."""
+    match), on the current stream; ``compact``: by the compacting forward; ``dense``: how its
+    dense output is taken (_DENSE)."""
     n = y0.shape[0]
     device = y0.device
     L = _lib.lib_for(spec)
@@ -1122,6 +1127,7 @@ def _forward_one(method, spec, y0, p, t1v, saveat_ts, cap, ws, kw, compact=False
         ts, ld, Kt = _ts_arg(saveat_ts, n)
         ys = (ws.ys if ok and ws.ys is not None and ws.ys.shape == (n, Kt, spec.dim)
               else torch.empty((n, Kt, spec.dim), dtype=torch.float64, device=device))
+        mode |= _DENSE[dense] if precision == "float64" else 0
         _lib.check(L.gs_fwd_record_saveat(_METHOD_CODE[method], spec.code, mode, n, _ptr(y0),
                                           _ptr(p), *args, _ptr(ts), ld, Kt, _ptr(ys),
                                           _stream()), "gs_fwd_record_saveat", L)
@@ -1184,6 +1190,47 @@ def _grow(method, spec, y0, p, t1v, saveat_ts, r0, streams, kw):
     return out
 
 
+# A planned tier is in the order of its cost, so the lanes that wait while one re-steps are few, and
+# the library's rule, set for batches in batch order, takes the pass apart at sizes where the
+# re-steps within the forward are faster; where depends on how long the longest trajectories are,
+# too.  Forward with 64 saved times and own end times, us, within / apart, K = 2, 4, 8: Van der Pol
+# 131,072 1813 / 1105, 1728 / 1069, 1749 / 1097, 700,000 2990 / 3739, 2914 / 3412, 2777 / 3528;
+# Lotka-Volterra 32,768 479 / 401, 472 / 397, 467 / 406, 131,072 664 / 811, 660 / 823, 680 / 844; Lorenz
+# 8192 326 / 285, 308 / 271, 320 / 275, 131,072 694 / 737, 690 / 749, 681 / 818; Lorenz-96 of 8 131,072
+# 1279 / 1686, 1282 / 1777, 1277 / 1927; Robertson 262,144 2497 / 2905, 2460 / 2835, 2415 / 2989; HIRES
+# 32,768 1321 / 1562, 1295 / 1568, 1282 / 1675.  So a plan of one tier times both, once per field,
+# interval, kind of batch and power of two of the size; several tiers overlap, and theirs is by
+# size (stiff Van der Pol, tiers of 122,252 and 8820 12.8 / 11.3 ms, 326,641 and 23,359 18.3 / 19.3).
+_DENSE_PLANNED: dict = {}  # (method, field key, K, uneven, K_times // 16, n.bit_length()) -> route
+DENSE_TUNE_MIN = 1 << 12   # (below, apart was the faster one everywhere: the library's rule)
+DENSE_TIER_MAX = 1 << 17
+DENSE_MARGIN = 0.01
+
+
+@_tuner
+def _time_dense(args) -> str:
+    ms = {}
+    for reps in (1, 2, 2):  # in turn; the first is to warm up
+        for route in ("within", "apart"):
+            t = _time_ms(lambda: _forward_one(*args, dense=route), reps)
+            ms[route] = t if reps == 1 else min(ms[route], t)
+    return "apart" if ms["apart"] < ms["within"] * (1.0 - DENSE_MARGIN) else "within"
+
+
+def _planned_dense(args, alone: bool) -> str:
+    """How the planned tier of _forward_one's arguments takes its dense output."""
+    method, spec, y0, _p, t1v, ts, cap, ws, kw = args
+    n = y0.shape[0]
+    if ts is None or kw["precision"] != "float64" or n < DENSE_TUNE_MIN:
+        return "auto"
+    if not alone:
+        return "within" if n > DENSE_TIER_MAX else "auto"
+    key = (method, spec.key, ws.ckpt_every, t1v is not None, ts.shape[-1] // 16, n.bit_length())
+    if key not in _DENSE_PLANNED:
+        _DENSE_PLANNED[key] = _time_dense(args)
+    return _DENSE_PLANNED[key]
+
+
 def _forward_planned(method, spec, y0, p, t1v, saveat_ts, ws: RecordSet, kw):
     """The tiers of ws, re-solved directly: every trajectory in the tier that held it last
     time, all tiers at once (side streams), overflowing rows re-solved afterwards."""
@@ -1202,9 +1249,12 @@ def _forward_planned(method, spec, y0, p, t1v, saveat_ts, ws: RecordSet, kw):
     kwp = kw
     if method == METHOD_ROS23 and kw["schedule"] == "auto":
         kwp = dict(kw, schedule="static")
-    launch = lambda rows, wsr: _forward_one(  # noqa: E731
-        method, spec, _take(y0, rows), _take(p, rows), _take(t1v, rows),
-        _take_ts(saveat_ts, rows), wsr.cap, wsr, kwp)
+
+    def launch(rows, wsr):
+        args = (method, spec, _take(y0, rows), _take(p, rows), _take(t1v, rows),
+                _take_ts(saveat_ts, rows), wsr.cap, wsr, kwp)
+        return _forward_one(*args, dense=_planned_dense(args, len(plan) == 1))
+
     out = [None] * len(plan)
     if all(st is None for st in streams):
         out = [(rows, launch(rows, wsr)) for rows, wsr in plan]

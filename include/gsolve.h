@@ -131,6 +131,14 @@ extern "C" {
 #define GS_OCC_ROS23_REVERSE 3 /* Rosenbrock23 reverse pass at K = 2 */
 #define GS_OCC_MIXED_REVERSE 4 /* Tsit5 float32-stage reverse pass at K = 2 */
 
+/* ORed into precision of gs_fwd_record_saveat (float64 with rec and ckpt): take the dense output as
+ * the trajectories are integrated, or by a kernel of its own from the checkpoints, instead of by
+ * the library's rule on sizes, which is set for batches in arbitrary order.  Results agree to
+ * rounding. */
+#define GS_SAVEAT_WITHIN 0x80000
+#define GS_SAVEAT_APART 0x100000
+#define GS_SAVEAT_MASK 0x180000
+
 /* per-trajectory status values written to status[] */
 #define GS_TRAJ_OK 0          /* reached t1 */
 #define GS_TRAJ_MAX_STEPS 1   /* max_steps attempts exhausted (or non-finite error) */
@@ -320,14 +328,16 @@ int gs_replay_saveat(int method, int field, int precision, long long n, const do
 /*
  * The adaptive forward with record (gs_tsit5_fwd_record / gs_ros23_fwd_record) that also
  * produces the dense output of gs_replay_saveat at the recording point: each requested time is
- * re-stepped from the start of the accepted step that brackets it, in float64 with rec and ckpt
- * by a second kernel from the checkpoints (a thread per few requested times), else as the
- * trajectory is integrated.  ys equals what gs_replay_saveat gives on the recorded mesh to
+ * re-stepped from the start of the accepted step that brackets it, as the trajectory is
+ * integrated, or, in float64 with rec and ckpt and at the sizes and intervals where that is
+ * faster (gs_abi.cu, states_apart), by a second kernel from the checkpoints (a thread per few
+ * requested times).  ys equals what gs_replay_saveat gives on the recorded mesh to
  * rounding (the same step function, compiled into another kernel).  Schedules: lanes refilled
  * from a work counter (GS_SCHED_REFILL, or AUTO when trajectories have their own end times and
  * are more than the chip holds at once; needs ckpt), persistent strided lanes
  * (GS_SCHED_STRIDED), one thread per trajectory otherwise (GS_SCHED_STATIC, or AUTO).  No
- * counterpart in the reference, whose saveat always replays the recorded mesh (gradsolve/warp/warp_replay.py:58-84).
+ * counterpart in the reference, whose saveat always replays the recorded mesh
+ * (gradsolve/warp/warp_replay.py:58-84).
  * method: GS_METHOD_TSIT5 (float64 or mixed) or GS_METHOD_ROS23 (float64).
  */
 int gs_fwd_record_saveat(int method, int field, int precision, long long n, const double* y0,
