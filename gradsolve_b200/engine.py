@@ -1204,7 +1204,7 @@ def _grow(method, spec, y0, p, t1v, saveat_ts, r0, streams, kw):
 _DENSE_PLANNED: dict = {}  # (method, field key, K, uneven, K_times // 16, n.bit_length()) -> route
 DENSE_TUNE_MIN = 1 << 12   # (below, apart was the faster one everywhere: the library's rule)
 DENSE_TIER_MAX = 1 << 17
-DENSE_MARGIN = 0.01
+DENSE_MARGIN = 0.03
 
 
 @_tuner
@@ -1471,6 +1471,42 @@ def _lanes_for(r, saveat: bool) -> int:
     return lanes if lanes and (r.method == METHOD_ROS23 or _few_steps(r)) else 0
 
 
+# With end times of their own, whether the split pass is the faster one depends on how much longer the
+# longest trajectories are than the others, us, lanes refilled / split: Robertson (t1 over a decade)
+# 50,000 1167 / 1740, with 32 saved times 1422 / 2546; with 32 saved times Lorenz 50,000 338 / 396,
+# 150,000 planned 543 / 863, Lotka-Volterra 150,000 planned 443 / 738; Van der Pol (above) the other way.
+# So from SPLIT_TUNE_MIN trajectories both passes are timed, once per field, kind of batch and power of
+# two of the size, on the first such record.
+SPLIT_TUNE_MIN = 1 << 12
+SPLIT_MARGIN = 0.03
+_SPLIT_PAYS: dict = {}  # (method, field key, saved times // 16, tiers, planned, bit_length) -> bool
+
+
+@_tuner
+def _time_split(run) -> bool:
+    ms = {}
+    for reps in (1, 2, 2):  # in turn; the first is to warm up
+        for split in (False, True):
+            t = _time_ms(lambda: run(split), reps)
+            ms[split] = t if reps == 1 else min(ms[split], t)
+    return ms[True] < ms[False] * (1.0 - SPLIT_MARGIN)
+
+
+def _split_pays(r, times: int, run) -> bool:
+    """Whether r's reverse pass, split or two-warp by its size, is the faster one (run(split) runs
+    it, or the unsplit one); by the size alone for batches of one end time, and under capture."""
+    if not r.uneven or r.n < SPLIT_TUNE_MIN:
+        return True
+    parts = _parts(r)
+    key = (r.method, r.spec.key, -(-times // 16), len(parts) > 1, parts[0][0] is not None,
+           r.n.bit_length())
+    if key not in _SPLIT_PAYS:
+        if torch.cuda.is_current_stream_capturing():
+            return True
+        _SPLIT_PAYS[key] = _time_split(run)
+    return _SPLIT_PAYS[key]
+
+
 def _adjoint_split(r: Record, lanes: int, p, ybar, ts, ysbar, want_y0, want_p, order,
                    work=None):
     L = _lib.lib_for(r.spec)
@@ -1517,15 +1553,20 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
             lanes = PAIRED
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
-    if lanes is not None:
-        res = _over_parts(r, lambda rr, rows: _adjoint_split(
-            rr, lanes, _take(p, rows), _take(ybar, rows).contiguous(), None, None, want_y0,
-            want_p, _lane_order(rr, rows is None)))
+
+    def run(split):
+        if split:
+            res = _over_parts(r, lambda rr, rows: _adjoint_split(
+                rr, lanes, _take(p, rows), _take(ybar, rows).contiguous(), None, None, want_y0,
+                want_p, _lane_order(rr, rows is None)))
+        else:
+            res = _over_parts(r, lambda rr, rows: _adjoint_one(
+                rr, _take(p, rows), _take(ybar, rows), want_y0=want_y0, want_p=want_p,
+                precision=precision, schedule=schedule, variant=variant,
+                in_batch_order=rows is None))
         return _scatter(r, res, 0), _scatter(r, res, 1)
-    res = _over_parts(r, lambda rr, rows: _adjoint_one(
-        rr, _take(p, rows), _take(ybar, rows), want_y0=want_y0, want_p=want_p,
-        precision=precision, schedule=schedule, variant=variant, in_batch_order=rows is None))
-    return _scatter(r, res, 0), _scatter(r, res, 1)
+
+    return run(lanes is not None and _split_pays(r, 0, run))
 
 
 def _window_order(a: torch.Tensor, b: Optional[torch.Tensor], window: int) -> torch.Tensor:
@@ -1722,19 +1763,23 @@ def adjoint_saveat(r, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
     per trajectory for an even one."""
     lanes = _lanes_for(r, True) if r.n and _split_applies(r, precision, schedule) else 0
     work = _split_work(r, ts.shape[-1] * (r.spec.dim + p.shape[1]), p.device) if lanes else None
-    if work is not None:
-        f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
-        res = _over_parts(r, lambda rr, rows: _adjoint_split(
-            rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
-            f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
-            work[id(rr)]))
-        return _scatter(r, res, 0), _scatter(r, res, 1)
     if schedule == "auto" and r.uneven and precision != "float32":
         schedule = "refill"  # (the float32 route runs one thread per trajectory)
-    res = _over_parts(r, lambda rr, rows: _adjoint_saveat_one(
-        rr, _take(p, rows), _take_ts(ts, rows), _take(ysbar, rows), _take(ybar, rows),
-        want_y0=want_y0, want_p=want_p, precision=precision, schedule=schedule))
-    return _scatter(r, res, 0), _scatter(r, res, 1)
+
+    def run(split):
+        if split:
+            f64 = lambda t: None if t is None else t.to(torch.float64).contiguous()  # noqa: E731
+            res = _over_parts(r, lambda rr, rows: _adjoint_split(
+                rr, lanes, _take(p, rows), f64(_take(ybar, rows)), _take_ts(ts, rows),
+                f64(_take(ysbar, rows)), want_y0, want_p, _lane_order(rr, rows is None),
+                work[id(rr)]))
+        else:
+            res = _over_parts(r, lambda rr, rows: _adjoint_saveat_one(
+                rr, _take(p, rows), _take_ts(ts, rows), _take(ysbar, rows), _take(ybar, rows),
+                want_y0=want_y0, want_p=want_p, precision=precision, schedule=schedule))
+        return _scatter(r, res, 0), _scatter(r, res, 1)
+
+    return run(work is not None and _split_pays(r, ts.shape[-1], run))
 
 
 def _adjoint_saveat_one(r: Record, p: torch.Tensor, ts: torch.Tensor, ysbar: torch.Tensor,
