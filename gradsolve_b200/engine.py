@@ -460,6 +460,8 @@ class RecordSet:
         if len(self.parts) == 1:  # one tier, whatever its rows' order: no host sync
             if self.uneven and self.n > WINDOW_UNEVEN:  # (the longest first over the batch)
                 return [torch.argsort(self.n_acc + self.n_rej, descending=True, stable=True)]
+            if not self.uneven and _ORDER_BATCH.get(_order_key(self.parts[0][1], self.n)):
+                return [torch.argsort(self.n_acc + self.n_rej, descending=True, stable=True)]
             return [_window_order(self.n_acc, self.n_rej, WINDOW_UNEVEN)]
         owner = torch.zeros(self.n, dtype=torch.int64, device=self.y_final.device)
         for k, (rows, _r) in enumerate(self.parts):
@@ -1566,7 +1568,10 @@ def adjoint(r, p: torch.Tensor, ybar: torch.Tensor, *, want_y0: bool = True,
                 in_batch_order=rows is None))
         return _scatter(r, res, 0), _scatter(r, res, 1)
 
-    return run(lanes is not None and _split_pays(r, 0, run))
+    split = lanes is not None and _split_pays(r, 0, run)
+    if not split:
+        _tune_order(r, schedule, lambda: run(False))
+    return run(split)
 
 
 def _window_order(a: torch.Tensor, b: Optional[torch.Tensor], window: int) -> torch.Tensor:
@@ -1585,9 +1590,61 @@ def prepare_lane_order(r) -> Optional[torch.Tensor]:
     first) on the current stream; the reverse pass picks it up.  Planned records (already ordered
     by cost) need none."""
     if isinstance(r, Record) and r.n >= ORDER_LANES_MIN:
-        r.lane_order = _window_order(r.n_acc, None, WINDOW_UNEVEN if r.uneven else WINDOW_EVEN)
+        whole = not r.uneven and _ORDER_BATCH.get(_order_key(r, r.n), False)
+        r.lane_order = _sorted_lanes(r, whole)
         return r.lane_order
     return None
+
+
+def _sorted_lanes(r, whole: bool) -> torch.Tensor:
+    if whole:
+        return torch.argsort(r.n_acc, descending=True, stable=True)
+    return _window_order(r.n_acc, None, WINDOW_UNEVEN if r.uneven else WINDOW_EVEN)
+
+
+# Windows order a warp's trajectories alone; a sort of the whole batch also starts the longest blocks
+# first, which decides where the blocks are a few waves and the counts spread, and scatters the
+# record's sectors, which decides above.  Reverse pass alone, us, windows of 512 / whole batch, whose
+# sort takes 65 us more: Van der Pol 30,000 304 / 230, 150,000 635 / 377, 400,000 1036 / 785, 2^20 2158
+# / 2106; Robertson 30,000 642 / 539, 150,000 1748 / 1457, 400,000 4047 / 4503; Lorenz-96 of 8 150,000
+# 1159 / 1012; Lotka-Volterra 30,000 113 / 108, 150,000 266 / 207, 400,000 552 / 491; Lorenz (t = 10)
+# 30,000 565 / 549, 150,000 1928 / 1889, 400,000 4962 / 5583.  So between these sizes both are timed with
+# their sorts, once per field, record type and power of two of the size, on the first record; a plan
+# of one tier goes by it.  The gradients are the same bits.
+_ORDER_BATCH: dict = {}  # _order_key -> the whole batch is sorted
+ORDER_TUNE = (1 << 14, 1 << 19)
+ORDER_MARGIN = 0.03
+
+
+def _order_key(r, n: int) -> tuple:
+    return r.method, r.spec.key, r.rec.element_size(), n.bit_length()
+
+
+@_tuner
+def _time_order(r, run) -> bool:
+    def once(whole):
+        r.lane_order = _sorted_lanes(r, whole)
+        run()
+
+    ms = {}
+    for reps in (1, 2, 2):  # in turn; the first is to warm up
+        for whole in (False, True):
+            t = _time_ms(lambda: once(whole), reps)
+            ms[whole] = t if reps == 1 else min(ms[whole], t)
+    return ms[True] < ms[False] * (1.0 - ORDER_MARGIN)
+
+
+def _tune_order(r, schedule: str, run) -> None:
+    """The lane order of batches like r's, and of r itself, the first time one comes (run() is its
+    reverse pass, one thread per trajectory)."""
+    if (not isinstance(r, Record) or r.uneven or schedule not in ("auto", "static") or
+            not ORDER_TUNE[0] <= r.n < ORDER_TUNE[1] or _IN_TUNER[0]):
+        return
+    key = _order_key(r, r.n)
+    if key in _ORDER_BATCH or torch.cuda.is_current_stream_capturing():
+        return
+    _ORDER_BATCH[key] = _time_order(r, run)
+    prepare_lane_order(r)
 
 
 # Trajectories per window of gs_lane_order: small ones keep a warp's checkpoint rows together; the
