@@ -1722,6 +1722,9 @@ class ReplayGraph:
         with torch.cuda.stream(side):  # one eager pass first: kernel attributes set, caches warm
             self._run()
         main.wait_stream(side)
+        # (the eager pass may have chosen another order, on its stream; the graph keeps this one
+        # alive, whatever order the record is given later)
+        self.order = prepare_lane_order(r)
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.out = self._run()
