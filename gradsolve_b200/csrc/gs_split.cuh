@@ -1,6 +1,7 @@
 // gs_split.cuh -- dense output and reverse passes split over threads where one thread per
 // trajectory leaves the chip idle: small batches and the few long trajectories of uneven ones
-// (float64, states of up to 3 components).
+// (float64; the saved states of every field with one thread per trajectory, the reverse pass
+// for states of up to 3 components).
 //
 // A trajectory's integration is a serial chain, but with its checkpoints recorded the work
 // around that chain is not:
@@ -18,10 +19,11 @@
 //     a chain G times shorter.
 // Step boundaries of the parts depend on the trajectory's step count and G alone, and the
 // states on neither K nor G, so gradients do not depend on the checkpoint interval or on which
-// other trajectories share the batch; against one thread per trajectory they agree to rounding.
+// other trajectories share the batch, at one G; another G, and one thread per trajectory, are
+// other evaluation orders of the same sums (gsolve.h says how far they agree).
 //
 // B200, stiff Van der Pol batch (20,011 trajectories, 2269 steps on average, 17,220 the longest,
-// 64 saved times): reverse pass 8.8 ms with one lane each, 1.6 ms with 16.
+// 64 saved times): reverse pass 8.9 ms with one lane each, 2.25 ms with 16.
 #pragma once
 #include <math_constants.h>
 

@@ -131,7 +131,7 @@ def choose_ckpt_every(policy, dim: int, n: int, cap: int, budget_bytes: Optional
 # free memory at a larger capacity, the first record takes that capacity: only the slots that
 # are written are touched, so the forward is as fast, and nothing is solved twice.  A small
 # share (2^18 trajectories of 3 components reach a sixteenth of 180 GB at 1780 steps), and what
-# the forward left unwritten is given back (fit_record).
+# all records alive hold beyond DEFAULT_CAP0 steps is bounded (fit_record).
 CAP_SHARE = 4  # of the checkpoint budget, itself a quarter of the free memory
 
 
